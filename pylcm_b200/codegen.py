@@ -10,6 +10,9 @@ Two kernels are generated per (regime, set of next-period targets):
     evaluated once per thread; only the mixed part runs in the inner loop.
     Infeasible actions are rejected before the continuation is touched.  The
     running (max, first argmax) is combined across lanes with warp shuffles.
+    Where the model's structure allows, the *line form* replaces the loop over
+    all actions (``RegimeKernels._line_plan``): bounds on groups of actions
+    rule most of them out, with the same result.
 
 ``lcm_expect_<tag>_<target>`` -- kernel (b), the shock expectation
     EV[k, col] = sum_j W[k, j] V'[j, col] / sum_j W[k, j]
@@ -97,9 +100,17 @@ def _c_float(v: float, ftype: str) -> str:
 
 
 class Emitter:
-    """Emits C statements for IR nodes, memoising node -> C expression."""
+    """Emits C statements for IR nodes, memoising node -> C expression.
 
-    def __init__(self, ftype: str, param_off: dict, provided: dict, prefix: str) -> None:
+    `fuse`: a sum or difference with a product is written as a fused
+    multiply-add (of the left product when both sides are one), the form the
+    compiler gives the same expression inside the search's plain loop.  Left to
+    itself it may choose differently where hoisting changes which product sits
+    in the loop, and near-ties of a float search then order differently."""
+
+    def __init__(self, ftype: str, param_off: dict, provided: dict, prefix: str, fuse: bool = False) -> None:
+        self.fuse = fuse
+        self.products: dict[int, tuple] = {}  # id(product node) -> its factors' C expressions
         self.ftype = ftype
         self.param_off = param_off  # flat name -> (offset, shape)
         self.vals: dict[int, str] = dict(provided)  # id(node) -> C expression
@@ -173,6 +184,15 @@ class Emitter:
                 xa, xb = self._arg(a, "f"), self._arg(b, "f")
             else:
                 xa, xb = self._arg(a), self._arg(b)
+            if self.fuse and n.dtype == "f":
+                if o == "*":
+                    self.products[id(n)] = (xa, xb)
+                elif o in "+-" and id(a) in self.products:
+                    p, q = self.products[id(a)]
+                    return self._tmp("f", f"lcm_fma({p}, {q}, {'-' if o == '-' else ''}({xb}))")
+                elif o in "+-" and id(b) in self.products:
+                    p, q = self.products[id(b)]
+                    return self._tmp("f", f"lcm_fma({'-' if o == '-' else ''}({p}), {q}, {xa})")
             if o in "+-*":
                 return self._tmp(n.dtype, f"{xa} {o} {xb}")
             if o == "/":
@@ -446,11 +466,11 @@ def _target_plan(tr: TracedRegime, tgt: RegimeSpec) -> TargetPlan:
 @dataclasses.dataclass(frozen=True)
 class LaunchConfig:
     block: int = 256
-    lanes: int = 1  # threads sharing one state (power of two <= 32)
+    lanes: int = 1  # threads sharing one state (power of two <= 32); line form: half of it
     chunk: int = 512  # actions per shared-memory table chunk
-    sb: int = 1  # states per thread (register blocking)
+    sb: int = 1  # states per thread (register blocking); line form: strips of a line per CTA
     min_blocks: int = 0  # __launch_bounds__ min CTAs per SM (0 = compiler's choice)
-    prune: bool = True  # single-precision search: exact skipping of action groups where eligible
+    prune: bool = True  # exact skipping of action groups where eligible (line form)
     # ... also in regimes with several continuous actions (measured slower than
     # the full search on the human-capital model: off unless asked for)
     prune_multi: bool = False
@@ -484,8 +504,10 @@ class RegimeKernels:
         order = sorted(targets, key=lambda s: (bool(s.states), s.rid))
         self.targets = [_target_plan(tr, t) for t in order] if not self.spec.terminal else []
         self._layout()
-        self._affine = self._affine_laws()
+        self._affine_all = self._affine_laws()
+        self._affine = self._affine_all if precision == "fp32" else {}
         self._groups = self._group_plan()
+        self._line = self._line_plan()
         tag_src = repr(
             (self.spec.name, [t.spec.name for t in self.targets], precision, dataclasses.astuple(cfg))
         )
@@ -639,13 +661,12 @@ class RegimeKernels:
         (state, discrete action) -- one fused multiply-add per action.  Its
         candidates are re-evaluated in double precision, so the search's
         rounding does not reach the published values beyond that search's
-        tolerance; the double-precision form keeps the law as written."""
+        tolerance; the double-precision form evaluates the law as written and
+        uses this one only to build the bounds of the line form."""
         out: dict = {}
-        if self.precision != "fp32":
-            return out
         dnames = {a.name for a in self.spec.actions if a.kind != "continuous"}
         for ti, t in enumerate(self.targets):
-            if t.scalar:
+            if t.scalar or t.unreachable:
                 continue
             for pos in t.cont_pos:
                 if t.spec.states[pos].grid.kind != "lin":
@@ -684,7 +705,7 @@ class RegimeKernels:
         of the bilinear read.  The candidates are re-evaluated in double
         precision as everywhere in this search."""
         spec = self.spec
-        if self.precision != "fp32" or not self.cfg.collapse or self._groups or spec.terminal:
+        if not self.cfg.collapse or self._groups or spec.terminal:
             return None
         if t.scalar or t.unreachable or len(t.cont_pos) != 2 or t.det_pos:
             return None
@@ -693,13 +714,13 @@ class RegimeKernels:
         cont_states = [a.name for a in spec.states if a.kind == "continuous"]
         names = [a.name for a in spec.actions]
         for cb, posB in enumerate(t.cont_pos):
-            if (ti, posB) not in self._affine:
+            if (ti, posB) not in self._affine_all:
                 continue
             ca, posA = 1 - cb, t.cont_pos[1 - cb]
             line = t.spec.states[posA].name
             if line not in cont_states:
                 continue
-            x0, g, cv = self._affine[(ti, posB)]
+            x0, g, cv = self._affine_all[(ti, posB)]
             ob = cv.args[1]
             kob = names.index(ob)
             if spec.actions[kob].size > self.COLLAPSE_MAX_OUTER:
@@ -831,6 +852,191 @@ class RegimeKernels:
         return {"axes": axes, "cons": cons, "acts": [a.name for a in cacts if a.name in used],
                 "scan": scan, "cacts": [a.name for a in cacts]}
 
+    # ------------------------------------------------------------ line form
+    LINE_MAX_ACTIONS = 2048  # continuous-action combinations held in shared memory
+    LINE_MAX_GROUPS = 512  # action groups held in shared memory
+    LINE_GROUP = 8  # actions per group
+    LINE_TESTS = 4  # group tests in flight per thread
+    LINE_BATCH = 4  # actions evaluated together per thread
+    LINE_MAX_SMEM = 100 * 1024  # of a CTA: two CTAs per SM
+
+    def _line_plan(self) -> dict | None:
+        """Eligibility and the affine pieces of the line form of kernel (a):
+        the exact search that skips action groups on bounds from
+        expectation rows held in shared memory.
+
+        A *line* is every state that differs in one continuous state only
+        (the line state); a CTA works on one line.  The expectation row of a
+        target does not depend on the line state, so the CTA holds it in
+        shared memory, with a windowed maximum beside it.  Consecutive
+        threads own consecutive states of the line, whose best actions lie
+        close together: a warp walks the union of its states' surviving
+        groups with little waste.
+
+        What bounds it: issue and the latency of dependent instructions (128
+        registers, 16 warps per SM); hence the group tests and the surviving
+        actions go several at a time without branches.  B200, one launch,
+        256 instances x 3500 states x 1000 actions in single precision: the
+        full search 1.9 ms, skipping per state with 4 scattered states per
+        thread 1.16 ms, the line form 0.52 ms (of it: surviving actions and
+        their re-evaluation 0.24, group tests 0.14, pilot 0.02, shared-memory
+        build 0.08).  Double precision, 48 x 2331 x 802: 0.26 -> 0.17 ms.  Two
+        axes, 2 x 1.6 M states x 900 actions: single 4.5 -> 2.3 ms, double
+        (1.6 M) 3.8 -> 2.2 ms.
+
+        Needed: a deterministic regime transition known per discrete action, a
+        utility free of the state, a state-free discount factor, and per
+        target either one continuous axis or two of which one collapses (see
+        `_collapse_info`), on linear grids, whose coordinate x = x0 + sum_k
+        coef_k a_k is affine in the continuous actions."""
+        spec, tr = self.spec, self.tr
+        if (not self.cfg.prune or spec.terminal or spec.taste_shocks or tr.regime_id is None or tr.beta is None
+                or not self.targets):
+            return None
+        cacts = [a for a in spec.actions if a.kind == "continuous"]
+        cstates = [a.name for a in spec.states if a.kind == "continuous"]
+        if not cacts or not cstates or (len(cacts) > 1 and self.cfg.prune_multi):
+            return None
+        cn = {a.name for a in cacts}
+        if any(k == "state" or (k == "action" and nm in cn) for k, nm in ir.const(tr.regime_id).deps()):
+            return None
+        U, beta = ir.const(tr.U), ir.const(tr.beta)
+        if not isinstance(U, ir.Expr) or any(k == "state" for k, _ in U.deps()):
+            return None
+        if not any(k == "action" and nm in cn for k, nm in U.deps()):
+            return None
+        if isinstance(beta, ir.Expr) and any(k in ("state", "action") for k, _ in beta.deps()):
+            return None
+        sizes = [a.size for a in cacts]
+        scan = cacts[int(np.argmax(sizes))].name
+        tg: dict[int, dict] = {}
+        line = None
+        for two in (True, False):  # the collapsed axes fix the line state
+            for ti, t in enumerate(self.targets):
+                if t.scalar or t.unreachable or t.det_pos or len(t.cont_pos) != (2 if two else 1):
+                    continue
+                coll = None
+                pos, ca = t.cont_pos[0], 0
+                if two:
+                    coll = self._collapse_info(ti, t)
+                    if coll is None or coll["ob"] == scan or (line is not None and coll["line"] != line):
+                        continue
+                    pos, ca = coll["posA"], coll["ca"]
+                ax = t.spec.states[pos]
+                if ax.grid.kind != "lin":
+                    continue
+                sp = _affine_split(ir.const(t.laws[ax.name].expr), cn)
+                if sp is None or scan not in sp[1]:
+                    continue
+                if two:
+                    line = coll["line"]
+                tg[ti] = {"pos": pos, "ca": ca, "x0": sp[0], "co": sp[1], "coll": coll}
+        if not tg:
+            return None
+        if line is None:
+            line = cstates[-1]
+        acts = [a.name for a in cacts if a.name == scan or any(a.name in x["co"] for x in tg.values())]
+        return {"targets": tg, "line": line, "kline": [a.name for a in spec.states].index(line),
+                "scan": scan, "kscan": [a.name for a in spec.actions].index(scan), "acts": acts,
+                "cacts": [a.name for a in cacts], "budget": self._scan_bound(scan)}
+
+    def _scan_bound(self, scan: str):
+        """The action-free side b of a constraint scan <= b (or <, or b >=
+        scan) in F: the scan action's grid being ascending, the actions that
+        meet it are a prefix of the grid.  None if F has no such
+        constraint."""
+        F = ir.const(self.tr.F)
+        stack = [F] if isinstance(F, ir.Expr) else []
+        while stack:
+            n = stack.pop()
+            if n.op == "and":
+                stack.extend(a for a in n.args if isinstance(a, ir.Expr))
+                continue
+            if n.op != "cmp" or n.args[0] not in ("<", "<=", ">", ">="):
+                continue
+            lhs, rhs = ir.const(n.args[1]), ir.const(n.args[2])
+            if n.args[0] in (">", ">="):
+                lhs, rhs = rhs, lhs
+            if not (lhs.op == "var" and tuple(lhs.args[:2]) == ("action", scan)):
+                continue
+            if rhs.dtype != "f" or any(k == "action" for k, _ in rhs.deps()):
+                continue
+            return rhs
+        return None
+
+    @property
+    def line_lanes(self) -> int:
+        """Threads sharing one state in the line form."""
+        return max(1, self.cfg.lanes // 2)
+
+    @property
+    def line_tile(self) -> int:
+        """States of one line that a CTA works on, a strip at a time."""
+        return self.cfg.sb * self.cfg.block // self.line_lanes
+
+    # (state, action) pairs of a batch from which the line form pays
+    LINE_MIN_PAIRS = 16_000_000
+
+    def line_config(self, n_items: int) -> LaunchConfig:
+        """The launch shape of kernel (a) for `n_items` instances where the
+        caller asks for none.
+
+        Small batches: the full search, whose threads per state fill the GPU
+        without the line form's per-CTA set-up (B200, milliseconds per solve
+        batch, full search / line form: 3500 states x 1000 actions, double
+        precision, 0.475 / 0.525; 31,500 x 450, two axes, 0.21 / 0.26 single
+        and 0.26 / 0.35 double; 21,000 x 1000: 1.33 / 0.90).  The
+        single-precision search over one continuous action keeps the line
+        form at every size (3500 x 1000: 0.71 / 0.68).
+
+        Threads per state: one, or more while the states do not fill the GPU
+        (21,000 states: 1 / 2 / 4 threads 1.34 / 0.95 / 0.90 ms; 70,000:
+        1.55 / 1.63 / 1.77).  Strips per CTA: a CTA that walks the whole line
+        builds its rows once, more CTAs fill the last wave better; the cheaper
+        of the two by waves x (strips + build), the build worth a third of a
+        strip, or two thirds with collapsed rows (280 lines of 500: 2 strips
+        2.18, 1 strip 2.70 ms; 140 lines: 1.82, 1.55)."""
+        cfg, spec = self.cfg, self.spec
+        if self._line is None:
+            return cfg
+        total = spec.n_states * n_items
+        one = len(self._line["cacts"]) == 1
+        if total * spec.n_actions < self.LINE_MIN_PAIRS and not (one and self.precision == "fp32"):
+            return dataclasses.replace(cfg, prune=False)
+        lanes = next((k for k, n in ((1, 60_000), (2, 30_000), (4, 12_000), (8, 6_000)) if total >= n), 16)
+        nline = spec.states[self._line["kline"]].size
+        lines = spec.n_states // nline * n_items
+        most = math.ceil(nline / (cfg.block // lanes))
+        build = 0.67 if any(x["coll"] for x in self._line["targets"].values()) else 0.35
+
+        def cost(k: int) -> float:
+            return math.ceil(lines * math.ceil(most / k) / (2 * 148)) * (k + build)
+
+        strips = min((k for k in (1, 2, 4) if k <= max(1, most)), key=cost)
+        return dataclasses.replace(cfg, lanes=2 * lanes, sb=strips)
+
+    def n_tiles(self) -> int:
+        """Tiles of kernel (a) per item."""
+        n = self.spec.n_states
+        if self._line is None:
+            return math.ceil(n / self.cfg.states_per_tile)
+        nline = self.spec.states[self._line["kline"]].size
+        return n // nline * math.ceil(nline / self.line_tile)
+
+    def _line_roots(self) -> list:
+        p = self._line
+        if not p:
+            return []
+        out = [ir.var("action", nm, "f") for nm in p["acts"]]
+        for x in p["targets"].values():
+            out.append(x["x0"])
+            out += list(x["co"].values())
+            if x["coll"] is not None:
+                out += [x["coll"]["x0"], x["coll"]["g"]]
+        if p["budget"] is not None:
+            out.append(p["budget"])
+        return out
+
     def _group_roots(self) -> list:
         g = self._groups
         if not g:
@@ -850,7 +1056,7 @@ class RegimeKernels:
         0 none, 1 per 16 columns (written by kernel (b)), 2 per GROUP_TILE
         tile of the two continuous axes (written by the statistics kernel)."""
         g = self._groups
-        if not g:
+        if not g or self._line is not None:
             return 0
         ti = next((i for i, x in enumerate(self.targets) if x is t), None)
         if ti is None or ti not in g["axes"]:
@@ -907,7 +1113,10 @@ class RegimeKernels:
         roots = [tr.F, tr.U]
         for x0, g, cv in getattr(self, "_affine", {}).values():
             roots += [x0, g, cv]
-        roots += self._group_roots() if getattr(self, "_groups", None) else []
+        if getattr(self, "_line", None):
+            roots += self._line_roots()
+        elif getattr(self, "_groups", None):
+            roots += self._group_roots()
         if tr.beta is not None:
             roots.append(tr.beta)
         if tr.regime_id is not None and self.targets:
@@ -995,9 +1204,14 @@ class RegimeKernels:
                 ni += 1
         NF, NI = max(nf, 1), max(ni, 1)
         B, LANES, CH, SB = cfg.block, cfg.lanes, cfg.chunk, cfg.sb
-        if self._groups:
+        line = self._line
+        if line is not None:
+            # a thread owns one state at a time; the CTA walks the strips of
+            # its part of the line
+            LANES, SB = self.line_lanes, 1
+        elif self._groups:
             CH = max(CH, self.GROUP_MAX_CHUNK)  # group skipping holds the whole table
-        SPT = cfg.states_per_tile
+        SPT = cfg.states_per_tile if line is None else self.line_tile
         SPB = B // LANES
         dstates = [a for a in spec.states if a.kind != "continuous"]
         NDS = max(len(dstates), 1)
@@ -1013,6 +1227,19 @@ class RegimeKernels:
                     cinfo[ti_] = c_
         rows_off = NF * CH * 4 + NI * CH * 4  # the collapsed rows follow the action table
         rows_bytes = max((2 * c["nob"] * c["namax"] * 4 for c in cinfo.values()), default=0)
+        TB = 4 if fp32 else 8  # bytes of a search value
+        if line is not None:
+            # the line form lays its shared memory out at run time: the whole
+            # continuous-action table, then the rows' windowed maxima and the
+            # rows
+            n_ac = spec.n_actions // ND
+            tab = (n_ac + 3) // 4 * 4 * (nf * TB + ni * 4)
+            rows_bytes = max((x["coll"]["nob"] if x["coll"] else 1) * self.targets[ti].spec.states[x["pos"]].size
+                             for ti, x in line["targets"].items()) * (12 if fp32 else 16)
+            line_bytes = tab + rows_bytes
+            if n_ac > self.LINE_MAX_ACTIONS or line_bytes > self.LINE_MAX_SMEM:
+                line_bytes = 0  # the kernel sees the shortage and runs the plain loop
+            rows_bytes = max(0, line_bytes - (NF * CH * TB + NI * CH * 4))
 
         L: list[str] = []
         ap = L.append
@@ -1070,6 +1297,12 @@ class RegimeKernels:
                 f"  __device__ __forceinline__ T F(int f) const {{ return (T)tabf[f * {CH} + j]; }}\n"
                 f"  __device__ __forceinline__ int I(int f) const {{ return tabi[f * {CH} + j]; }} }};"
             )
+        if line is not None:
+            ap(
+                f"struct AFLine_{self.tag} {{ {TT} v[{NF}]; const int* vi; const {TT}* R;\n"
+                f"  __device__ __forceinline__ {TT} F(int f) const {{ return v[f]; }}\n"
+                f"  __device__ __forceinline__ int I(int f) const {{ return vi[f]; }} }};"
+            )
         ap(
             f"struct AFLoc_{self.tag} {{ double v[{NF}]; int vi[{NI}];\n"
             f"  __device__ __forceinline__ double F(int f) const {{ return v[f]; }}\n"
@@ -1081,7 +1314,12 @@ class RegimeKernels:
         # the selected target (TSEL < 0: all targets by probability / id)
         proc_names = [a.name for a in spec.states if a.kind == "process"]
 
-        def sa_body(T: str, E: str, tsel: int, sim: bool = False, coll: dict | None = None) -> list[str]:
+        def sa_body(T: str, E: str, tsel: int, sim: bool = False, coll: dict | None = None,
+                    fast: bool = False) -> list[str]:
+            """`fast`: no branches -- an infeasible action is evaluated too
+            (the caller reads `ok_`), and the interpolation leaves out the
+            zero-safe rule, so a result that is not finite is to be redone
+            with the plain form."""
             prov = pv()
             for i, n in enumerate(bP):
                 prov[id(n)] = _cast(f"PVd[{i}]", n.dtype, T)
@@ -1103,12 +1341,12 @@ class RegimeKernels:
                 prov[id(ir.var("state", a.name, "i"))] = f"SI[{i}]"
             for a in dacts:
                 prov[id(ir.var("action", a.name, "i"))] = f"DI_{a.name}"
-            e = Emitter(T, self.param_off, prov, "q")
+            e = Emitter(T, self.param_off, prov, "q", fuse=fast)
             out: list[str] = []
             fexpr = e.emit(self.tr.F)
             out += e.lines
             e.lines = []
-            out.append(f"if (!({fexpr})) return false;")
+            out.append(f"const bool ok_ = {fexpr};" if fast else f"if (!({fexpr})) return false;")
             uexpr = e.emit(self.tr.U)
             out += e.lines
             e.lines = []
@@ -1199,8 +1437,10 @@ class RegimeKernels:
                         if kind == "lin" and not sim and (ti, pos) in affine_names:
                             # (x0 + g c - a) b as K + M c: K, M are loop-invariant
                             x0n, gn, cvn = affine_names[(ti, pos)]
-                            cc = (f"((({T})({x0n}) - C.a{ti}_{ci}) * C.b{ti}_{ci} + "
-                                  f"(({T})({gn}) * C.b{ti}_{ci}) * ({T})({cvn}))")
+                            K = f"(({T})({x0n}) - C.a{ti}_{ci}) * C.b{ti}_{ci}"
+                            M = f"({T})({gn}) * C.b{ti}_{ci}"
+                            cc = (f"lcm_fma({M}, ({T})({cvn}), {K})" if coll is not None
+                                  else f"({K} + ({M}) * ({T})({cvn}))")
                         elif kind == "lin":
                             cc = f"lcm_coord_lin<{T}>(({T})({x}), C.a{ti}_{ci}, C.b{ti}_{ci})"
                         elif kind == "log":
@@ -1213,7 +1453,7 @@ class RegimeKernels:
                     rows = [] if multi else [("row", off)] + ([("rowh", off_hi)] if off_hi is not None else [])
                     if coll is not None and ti == coll["ti"]:
                         rows = []
-                        inner.append(f"{T} ev = lcm_interp1s<{T}>(AF.R, C.n{ti}_{coll['posA']}, c{coll['ca']});")
+                        inner.append(f"{T} ev = lcm_interp1s{'f' if fast else ''}<{T}>(AF.R, C.n{ti}_{coll['posA']}, c{coll['ca']});")
                     if multi:
                         inner.append(f"{T} ev = ({T})0;")
                         inner += self._sim_extrapolated_expectation(ti, t, T, E, None, proc_names, dn, mk)
@@ -1247,7 +1487,8 @@ class RegimeKernels:
                 # a negative weight poisons the row even when the weights sum
                 # to exactly one (Q_and_F.py:1401-1432, 646-653)
                 out.append(f"ce = valid ? ((mass == ({T})1) ? ce : ce / mass) : lcm_lim<{T}>::nan();")
-            out.append(f"Q = ({T})({uexpr}) + ({T})({bexpr}) * ce;")
+            out.append(f"Q = lcm_fma(({T})({bexpr}), ce, ({T})({uexpr}));" if coll is not None
+                       else f"Q = ({T})({uexpr}) + ({T})({bexpr}) * ce;")
             return out
 
         di_params = "".join(f"int DI_{a.name}, " for a in dacts)
@@ -1273,6 +1514,32 @@ class RegimeKernels:
             for s_ in sa_body("T", "E", ti_, coll=c_):
                 ap("  " + s_)
             ap("  return true;\n}")
+
+        for ti_, x_ in (line["targets"].items() if line is not None else ()):
+            if x_["coll"] is not None:
+                continue
+            # target ti_ read from its expectation row in shared memory (R)
+            ap(
+                f"template <typename T, typename E, typename AFN>\n"
+                f"__device__ __forceinline__ bool lcm_sl{ti_ + 1}_{self.tag}(const Ctx_{self.tag}<T, E>& C, "
+                f"const double* __restrict__ PV, const double* PVd, const double* DV, const double* SV, "
+                f"const double* SDV, const AFN& AF, const int* SI, {di_params}int period, double age, T& Q) {{"
+            )
+            for s_ in sa_body("T", "E", ti_, coll={"ti": ti_, "ca": 0, "cb": -1, "posA": x_["pos"]}):
+                ap("  " + s_)
+            ap("  return true;\n}")
+        for ti_, x_ in (line["targets"].items() if line is not None else ()):
+            # the branch-free form of target ti_'s evaluation
+            ap(
+                f"template <typename T, typename E, typename AFN>\n"
+                f"__device__ __forceinline__ bool lcm_sf{ti_ + 1}_{self.tag}(const Ctx_{self.tag}<T, E>& C, "
+                f"const double* __restrict__ PV, const double* PVd, const double* DV, const double* SV, "
+                f"const double* SDV, const AFN& AF, const int* SI, {di_params}int period, double age, T& Q) {{"
+            )
+            rd = {"ti": ti_, "ca": 0, "cb": -1, "posA": x_["pos"]} if x_["coll"] is None else x_["coll"]
+            for s_ in sa_body("T", "E", ti_, coll=rd, fast=True):
+                ap("  " + s_)
+            ap("  return ok_;\n}")
 
         ap(
             f"template <typename T, typename E, typename AFN>\n"
@@ -1346,7 +1613,14 @@ class RegimeKernels:
         ap(f"    const int n_ac = n_actions / {ND};")
         ap(f"    const double* __restrict__ atf = lcm_wp<const double>(it, {self.W_ATAB});")
         ap(f"    const int* __restrict__ ati = reinterpret_cast<const int*>(atf + (i64){nf} * n_actions);")
-        ap(f"    const int sbase = (tile - tile_prefix[item]) * {SPT} + (int)threadIdx.x / {LANES};")
+        if line is None:
+            ap(f"    const int sbase = (tile - tile_prefix[item]) * {SPT} + (int)threadIdx.x / {LANES};")
+        else:
+            ap(f"    const int nLine = lcm_wi(it, {self.W_SSIZE + line['kline']});")
+            ap(f"    const int ppl = (nLine + {SPT - 1}) / {SPT};  // parts of a line")
+            ap("    const int line_id = (tile - tile_prefix[item]) / ppl;")
+            ap(f"    const int part0 = (tile - tile_prefix[item] - line_id * ppl) * {SPT};")
+            ap('    unsigned dyn_smem; asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(dyn_smem));')
         ap(f"    const int lane = (int)threadIdx.x % {LANES};")
         ap("    (void)period; (void)age; (void)ati; (void)PV;")
         for s_ in eP.lines:
@@ -1356,7 +1630,13 @@ class RegimeKernels:
             ap(f"    PVd[{i}] = (double)({v});")
         if not bP:
             ap("    PVd[0] = 0.0;")
+        if line is not None:
+            ap(f"    for (int strip = 0; strip < {cfg.sb}; ++strip) {{")
+            ap(f"    const int pos0 = part0 + strip * {SPB};")
+            ap("    if (pos0 >= nLine) break;  // uniform over the CTA")
         ap(f"    int SI[{SB}][{NDS}]; double SV[{SB}][{nS}]; bool act[{SB}]; int sidx[{SB}];")
+        if line is not None:
+            cinfo_rows, cinfo = cinfo, {}  # the rows are read by the line form only
         kline = next(iter(cinfo.values()))["kline"] if cinfo else -1
         if cinfo:
             # states walked with the line state fastest (a tile then covers at
@@ -1365,20 +1645,28 @@ class RegimeKernels:
             ap(f"    const int nLine = lcm_wi(it, {self.W_SSIZE + kline});")
             ap(f"    const int line0 = ((tile - tile_prefix[item]) * {SPT}) / nLine;")
         ap(f"    #pragma unroll\n    for (int kb = 0; kb < {SB}; ++kb) {{")
-        ap(f"      const int s = sbase + kb * {SPB};")
-        ap("      act[kb] = s < n_states; sidx[kb] = s;")
-        ap("      int srem = act[kb] ? s : 0;")
         order = list(range(len(spec.states) - 1, -1, -1))
+        if line is None:
+            ap(f"      const int s = sbase + kb * {SPB};")
+            ap("      act[kb] = s < n_states; sidx[kb] = s;")
+            ap("      int srem = act[kb] ? s : 0;")
+        else:
+            ap(f"      const int pos = pos0 + (int)threadIdx.x / {LANES};")
+            ap("      act[kb] = pos < nLine;")
+            ap(f"      const int si_{spec.states[line['kline']].name} = act[kb] ? pos : nLine - 1;")
+            ap("      int srem = line_id;")
+            order = [k for k in order if k != line["kline"]]
         if cinfo:
             order = [kline] + [k for k in order if k != kline]
         for k in order:
             ax = spec.states[k]
             ap(f"      const int si_{ax.name} = srem % lcm_wi(it, {self.W_SSIZE + k}); srem /= lcm_wi(it, {self.W_SSIZE + k});")
-        if cinfo:
+        if cinfo or line is not None:
             phys = "0"
             for k, ax in enumerate(spec.states):
                 phys = f"({phys}) * lcm_wi(it, {self.W_SSIZE + k}) + si_{ax.name}"
-            ap(f"      if (act[kb]) sidx[kb] = {phys};")
+            ap(f"      {'sidx[kb]' if line is not None else 'if (act[kb]) sidx[kb]'} = {phys};")
+        if cinfo:
             ap("      lslot[kb] = act[kb] ? s / nLine - line0 : 0;")
         for k, ax in enumerate(spec.states):
             if ax.kind == "continuous":
@@ -1400,8 +1688,11 @@ class RegimeKernels:
         else:
             ap(f"    {BEST}<{ST}> best[{SB}];")
             ap(f"    #pragma unroll\n    for (int kb = 0; kb < {SB}; ++kb) best[kb].init();")
+        if line is not None:
+            for s_ in self._line_prefix_lines(bP, bS, ST):
+                ap("    " + s_)
         # ---- discrete-action loop (unrolled: ND is a compile-time constant)
-        ap(f"    #pragma unroll\n    for (int ad = 0; ad < {ND}; ++ad) {{")
+        ap(f"    #pragma unroll{' 1' if line is not None else ''}\n    for (int ad = 0; ad < {ND}; ++ad) {{")
         dl: list[str] = []
         decode_disc(dl, "ad")
         for s_ in dl:
@@ -1417,7 +1708,7 @@ class RegimeKernels:
         ap(f"      #pragma unroll\n      for (int kb = 0; kb < {SB}; ++kb) {{")
         if bSD:
             # re-derive the state variables of slot kb for the SD phase
-            ap("        int srem = act[kb] ? sidx[kb] : 0;")
+            ap(f"        int srem = {'sidx[kb]' if line is not None else 'act[kb] ? sidx[kb] : 0'};")
             for k in range(len(spec.states) - 1, -1, -1):
                 ax = spec.states[k]
                 ap(f"        const int si_{ax.name} = srem % lcm_wi(it, {self.W_SSIZE + k}); srem /= lcm_wi(it, {self.W_SSIZE + k});")
@@ -1898,6 +2189,25 @@ class RegimeKernels:
             o.append("}")
             return o
 
+        def line_info(ti: int) -> dict | None:
+            """Kernel-scope expressions of the line plan of target ti (None:
+            the plan does not cover it)."""
+            x = line["targets"].get(ti) if line is not None else None
+            if x is None:
+                return None
+            ia = {id(n): i for i, n in enumerate(bA)}
+            f = lambda n: slot[ia[id(n)]][1]  # noqa: E731
+            t = self.targets[ti]
+            key = "0"
+            for kind, name, size in t.key_vars:
+                iv = f"SI[0][{[a.name for a in dstates].index(name)}]" if kind == "state" else f"DI_{name}"
+                key = f"({key}) * {size} + {iv}"
+            return {"x": x, "uf": f(ir.const(self.tr.U)),
+                    "avf": {nm: f(ir.var("action", nm, "f")) for nm in line["acts"]},
+                    "beta": provider(ir.const(self.tr.beta), "0"), "x0": provider(ir.const(x["x0"]), "0"),
+                    "co": {nm: provider(ir.const(c), "0") for nm, c in x["co"].items()}, "key": key,
+                    "B": None if x["coll"] is None else tuple(provider(ir.const(x["coll"][k]), "0") for k in ("x0", "g"))}
+
         any_pruned = False
         n_gacts = 0
         if unswitch:
@@ -1909,11 +2219,20 @@ class RegimeKernels:
             for ti, t in enumerate(self.targets):
                 ap(f"      {'if' if first else 'else if'} (rid == {t.spec.rid}) {{")
                 first = False
-                gi = group_info(ti)
+                gi = group_info(ti) if line is None else None
                 if gi is not None:
                     any_pruned = True
                     n_gacts = max(n_gacts, len(GP["acts"]))
-                if ti in cinfo:
+                li = line_info(ti)
+                if li is not None:
+                    fn = f"lcm_sl{ti + 1}_{self.tag}"
+                    if li["x"]["coll"] is not None:
+                        fn = f"lcm_sc{ti + 1}_{self.tag}" if fp32 else SA.format(ti + 1)
+                    di_args = "".join(f"DI_{a.name}, " for a in dacts)
+                    call = f"{fn}<{ST}, {ST}>(C, PV, PVd, DV, SV[0], SDV[0], af, SI[0], {di_args}period, age, q)"
+                    fast = call.replace(fn, f"lcm_sf{ti + 1}_{self.tag}", 1)
+                    body = self._line_loop(ti, li, call, fast, inner_loop(SA.format(ti + 1)), nf, ni)
+                elif ti in cinfo:
                     body = inner_loop_collapse(ti, cinfo[ti])
                 else:
                     body = inner_loop(SA.format(ti + 1)) if gi is None else inner_loop_groups(SA.format(ti + 1), gi)
@@ -1928,9 +2247,13 @@ class RegimeKernels:
             for s_ in inner_loop(SA.format(0)):
                 ap("      " + s_)
         ap("    }")
+        if line is not None:
+            L.insert(gumax_at, f"  __shared__ float4 gI[{self.LINE_MAX_GROUPS}]; __shared__ int gWin, gLook;"
+                     + ("" if fp32 else f" __shared__ int gAbs[{self.COLLAPSE_MAX_OUTER}];"))
         if any_pruned:
             L.insert(gumax_at, f"  __shared__ float gU[{GMAX}], gLo[{max(n_gacts, 1) * GMAX}], gHi[{max(n_gacts, 1) * GMAX}];")
-        self.prunes_groups = any_pruned
+        # exact skipping by the single-precision group plan (either loop form)
+        self.prunes_groups = any_pruned or (line is not None and bool(self._groups))
 
         # ---- reduction and epilogue
         def final_eval(a_var: str, out_var: str, loc: str) -> list[str]:
@@ -2018,6 +2341,8 @@ class RegimeKernels:
             ap("        Vout[s] = v; Pout[s] = pol;")
         ap("      }")
         ap("    }")
+        if line is not None:
+            ap("    }  // strips")
         ap("  }")
         ap("}")
         self.smem_bytes = NF * CH * (4 if fp32 else 8) + NI * CH * 4 + rows_bytes
@@ -2068,6 +2393,315 @@ class RegimeKernels:
         ap("}")
         L += self._sim_kernel(locals())
         return "\n".join(L)
+
+    def _line_prefix_lines(self, bP: list, bS: list, ST: str) -> list[str]:
+        """Per state: `jfe`, the number of scan-action grid points that can
+        meet the budget constraint (the whole grid without one), by the same
+        comparison in the search's type, and `thr`, the running threshold."""
+        p = self._line
+        o = [f"const int gN = lcm_wi(it, {self.W_ASIZE + p['kscan']});",
+             f"{ST} thr = -lcm_lim<{ST}>::inf();",
+             "int jfe = act[0] ? gN : 0;"]
+        b = p["budget"]
+        if b is not None:
+            expr = None
+            if b.op == "const":
+                expr = _c_float(float(b.args[0]), "double")
+            for lst, fmt in ((bP, "PVd[{i}]"), (bS, "SV[0][{i}]")):
+                for i, m in enumerate(lst):
+                    if m is b:
+                        expr = fmt.format(i=i)
+            if expr is not None:
+                o += ["{",
+                      f"  const double* sg = lcm_wp<const double>(it, {self.W_AGRID + p['kscan']});",
+                      f"  const {ST} bound = ({ST})({expr});",
+                      "  int lo = 0, hi = jfe;",
+                      f"  while (lo < hi) {{ const int mid = (lo + hi) >> 1; if (({ST})sg[mid] <= bound) lo = mid + 1; else hi = mid; }}",
+                      "  jfe = lo;",
+                      "}"]
+        o.append("const int jfw = __reduce_max_sync(0xffffffffu, jfe);")
+        return o
+
+    def _line_loop(self, ti: int, li: dict, call: str, fast: str, plain: list[str], nf: int, ni: int) -> list[str]:
+        """The line form's loop over the continuous actions of one discrete
+        action toward target ti (one strip of states, `LANES` threads each).
+
+        A group is a run of G consecutive values of the scan action with the
+        other continuous actions fixed (a combination o_).  Its Q values are
+        bounded by its largest utility plus beta times the largest entry of
+        the expectation row among the nodes its coordinates can reach, plus
+        eight float roundings of either term; it is skipped when that is
+        below the state's running second best (best in double precision), or
+        the second best of a few spread pilot actions.  Utility and
+        coordinate ranges, row maxima and the bound are float in both
+        precisions (rounded up from double); coordinates are widened by 0.02
+        plus a cover of the law's rounding.  Groups that reach beyond the
+        grid, and NaN bounds, are never skipped.
+
+        `fast` evaluates an action without branches, `call` with the
+        zero-safe rule.  In double precision with a collapsed axis `fast`
+        reads the collapsed row, an ulp or so away from the bilinear read of
+        `call`: it only rules actions out, `call` decides."""
+        fp32 = self.precision == "fp32"
+        ST = "float" if fp32 else "double"
+        p, x = self._line, li["x"]
+        coll = x["coll"]
+        verify = coll is not None and not fp32
+        B, LANES = self.cfg.block, self.line_lanes
+        G = max(self.LINE_GROUP, LANES)
+        anames = [a.name for a in self.spec.actions]
+        kscan = p["kscan"]
+        later = list(range(kscan + 1, len(anames)))
+        others = [nm for nm in x["co"] if nm != p["scan"]]
+        multi = len(p["cacts"]) > 1
+        ninf = f"-lcm_lim<{ST}>::inf()"
+        TB = 4 if fp32 else 8
+        nrow = coll["nob"] if coll else 1
+        A_, Bs = f"(float)C.a{ti}_{x['ca']}", f"(float)C.b{ti}_{x['ca']}"
+        fmin_, fmax_, fabs_ = ("fminf", "fmaxf", "fabsf") if fp32 else ("fmin", "fmax", "fabs")
+        up_ = "" if fp32 else "__double2float_ru"
+        o = ["{",
+             f"const int nA = C.n{ti}_{x['pos']};",
+             f"const float beta_b = (float)({li['beta']});"]
+        if later:
+            o.append("const int gS = " + " * ".join(f"lcm_wi(it, {self.W_ASIZE + k})" for k in later) + ";")
+        else:
+            o.append("const int gS = 1;")
+        o += [f"const int gpc = (gN + {G - 1}) / {G};",
+              "const int ncomb = gN > 0 ? n_ac / gN : 0;",
+              f"const int rows_at = ((n_ac + 3) & ~3) * {nf * TB + ni * 4};",
+              "// uniform over the CTA (one item per tile)",
+              f"const bool lf = beta_b >= 0.0f && n_ac <= {self.LINE_MAX_ACTIONS} && ncomb * gpc <= {self.LINE_MAX_GROUPS} "
+              f"&& gN >= {2 * G} && nA >= 2 && (unsigned)(rows_at + {nrow * (8 + TB)} * nA) <= dyn_smem"
+              + (f" && C.n{ti}_{coll['posB']} >= 2 && lcm_wi(it, {self.W_ASIZE + coll['kob']}) == {nrow}" if coll else "")
+              + ";",
+              "if (!lf) {"]
+        o += ["  " + s for s in plain]
+        o.append("} else {")
+        b: list[str] = []
+        # shared memory: the action table (a row of columns per action), the
+        # integer columns, the windowed (maximum, largest finite magnitude)
+        # of the rows, the rows
+        b += [f"{ST}* ltab = reinterpret_cast<{ST}*>(lcm_smem);",
+              f"int* lti = reinterpret_cast<int*>(lcm_smem + ((n_ac + 3) & ~3) * {nf * TB});",
+              "float2* mw = reinterpret_cast<float2*>(lcm_smem + rows_at);",
+              f"{ST}* row = reinterpret_cast<{ST}*>(mw + {nrow} * nA);",
+              f"const float gM = (float)({li['co'][p['scan']]}) * {Bs};",
+              # with one discrete action the strips of a tile share everything
+              f"if ({'strip == 0' if self.spec.n_discrete_actions == 1 else 'true'}) {{",
+              "__syncthreads();  // the previous tile's, strip's or action's reads are done",
+              f"for (int j = threadIdx.x; j < n_ac; j += {B}) {{",
+              "  const i64 a = (i64)ad * n_ac + j;"]
+        for k in range(nf):
+            b.append(f"  ltab[j * {nf} + {k}] = ({ST})atf[(i64){k} * n_actions + a];")
+        for k in range(ni):
+            b.append(f"  lti[j * {ni} + {k}] = ati[(i64){k} * n_actions + a];")
+        b += ["}",
+              "if (threadIdx.x == 0) {",
+              "  // a group reaches at most wd nodes (on an evenly spaced scan grid): two",
+              "  // windows cover it, or more of the largest window; a group that reaches",
+              "  // further is not skipped",
+              f"  const double* sg = lcm_wp<const double>(it, {self.W_AGRID + kscan});",
+              f"  const float wd = fabsf(gM) * (float)((sg[gN - 1] - sg[0]) / (gN - 1)) * {float(G - 1)}f + 2.1f;",
+              "  int w = 2;",
+              "  while (w < 32 && 2 * w < wd) w <<= 1;",
+              "  gWin = w; gLook = wd < 1e4f ? max(2, (int)ceilf(wd / w)) : 2;",
+              "}"]
+        if verify:
+            b.append(f"if (threadIdx.x < {nrow}) gAbs[threadIdx.x] = 0;")
+        if coll:
+            cb = coll["cb"]
+            b += [f"const int nB = C.n{ti}_{coll['posB']};",
+                  f"const double* obg = lcm_wp<const double>(it, {self.W_AGRID + coll['kob']});",
+                  f"const {ST}* blk = C.ev{ti} + (i64)({li['key']}) * ((i64)nA * nB);",
+                  f"for (int e = threadIdx.x; e < {nrow} * nA; e += {B}) {{",
+                  "  const int w = e % nA, ob = e / nA;",
+                  f"  const {ST} cB = ((({ST})({li['B'][0]})) - C.a{ti}_{cb}) * C.b{ti}_{cb} + "
+                  f"((({ST})({li['B'][1]})) * C.b{ti}_{cb}) * ({ST})obg[ob];",
+                  f"  {ST} fB; const int lB = lcm_lower(cB, nB, fB); const {ST} uB = cB - fB;"]
+            if cb == 1:
+                b.append(f"  const {ST} va = blk[(i64)w * nB + lB], vb = blk[(i64)w * nB + lB + 1];")
+            else:
+                b.append(f"  const {ST} va = blk[(i64)lB * nA + w], vb = blk[(i64)(lB + 1) * nA + w];")
+            b += [f"  {ST} val = va + uB * (vb - va);",
+                  f"  if (!lcm_isfinite(val)) val = lcm_zs(({ST})1 - uB, va) + lcm_zs(uB, vb);",
+                  "  row[e] = val;",
+                  "}"]
+        else:
+            b += [f"const {ST}* src = C.ev{ti} + (i64)({li['key']}) * nA;",
+                  f"for (int e = threadIdx.x; e < nA; e += {B}) row[e] = __ldg(src + e);"]
+        b += ["__syncthreads();",
+              "const int win = gWin;",
+              f"for (int e = threadIdx.x; e < {nrow} * nA; e += {B}) {{",
+              "  const int lim = min(win, nA - e % nA);",
+              f"  {ST} m = row[e], a = lcm_isfinite(m) ? {fabs_}(m) : ({ST})0;"]
+        if verify:
+            b.append("  atomicMax(&gAbs[e / nA], __float_as_int(__double2float_ru(a)));")
+        b += ["  #pragma unroll 4\n  for (int k = 1; k < lim; ++k) {",
+              f"    const {ST} v = row[e + k];",
+              "    m = lcm_nanmax(m, v);",
+              f"    a = {fmax_}(a, lcm_isfinite(v) ? {fabs_}(v) : ({ST})0);",
+              "  }",
+              f"  mw[e] = make_float2({up_}(m), {up_}(a));",
+              "}",
+              f"for (int g = threadIdx.x; g < ncomb * gpc; g += {B}) {{",
+              f"  const int o_ = g / gpc, i0 = (g - o_ * gpc) * {G};",
+              "  const int jb = (o_ / gS) * gN * gS + (o_ % gS) + i0 * gS;",
+              f"  const int m = min({G}, gN - i0);",
+              f"  {ST} um = ltab[jb * {nf} + {li['uf']}];",
+              f"  for (int t = 1; t < m; ++t) um = lcm_nanmax(um, ltab[(jb + t * gS) * {nf} + {li['uf']}]);",
+              f"  gI[g] = make_float4({up_}(um), (float)ltab[jb * {nf} + {li['avf'][p['scan']]}], "
+              f"(float)ltab[(jb + (m - 1) * gS) * {nf} + {li['avf'][p['scan']]}], 0.0f);",
+              "}",
+              "__syncthreads();",
+              "}  // shared-memory build",
+              "const int win = gWin, nlk = gLook;",
+              f"const float gx = (float)({li['x0']});",
+              f"const float gK0 = (gx - {A_}) * {Bs};",
+              f"const float gE0 = (fabsf(gx) + fabsf({A_})) * fabsf({Bs});"]
+        # per combination of the other continuous actions
+        b.append("for (int o_ = 0; o_ < ncomb; ++o_) {")
+        c: list[str] = ["const int jb0 = (o_ / gS) * gN * gS + (o_ % gS);"]
+        if coll:
+            ostr = " * ".join(f"lcm_wi(it, {self.W_ASIZE + k})" for k in range(coll["kob"] + 1, len(anames))) or "1"
+            c += [f"const int obi = (jb0 / ({ostr})) % {nrow};",
+                  f"const {ST}* rrow = row + obi * nA; const float2* mrow = mw + obi * nA;"]
+        else:
+            c.append(f"const {ST}* rrow = row; const float2* mrow = mw;")
+        if verify:
+            c.append(f"const double babs = (double)beta_b * (double)__int_as_float(gAbs[obi]);")
+        c.append("const float4* grp = gI + o_ * gpc;")
+        c.append("float gK = gK0, gE = gE0 + fabsf(gM) * fmaxf(fabsf(grp[0].y), fabsf(grp[gpc - 1].z));")
+        for nm in others:
+            c.append(f"{{ const float v = ((float)({li['co'][nm]}) * {Bs}) * (float)ltab[jb0 * {nf} + {li['avf'][nm]}]; "
+                     "gK += v; gE += fabsf(v); }")
+        c += ["gE = 0.02f + 4e-6f * gE;  // cover of the coordinate's rounding in the search",
+              "const float gTop = (float)(nA - 1);"]
+
+        def load(j: str) -> list[str]:
+            if nf == 2:
+                v = f"const {ST}2 lv = reinterpret_cast<const {ST}2*>(ltab)[{j}];"
+                vals = "lv.x, lv.y"
+            else:
+                v = f"const {ST}* lv = ltab + {j} * {nf};"
+                vals = ", ".join(f"lv[{k}]" for k in range(nf))
+            return [v, f"const AFLine_{self.tag} af{{{{{vals}}}, lti + {j} * {ni}, rrow}};"]
+
+        ev = load("j") + [f"{ST} q;"]
+        # pilot: a few spread actions of the feasible prefix give a first
+        # threshold (distinct actions, so never above the final second best)
+        up = "if (ok && q > p2) { if (q > p1) { p2 = p1; p1 = q; pb = si; } else p2 = q; }"
+        c.append("{")
+        c.append(f"  {ST} p1 = {ninf}, p2 = {ninf}; int pb = 0; (void)pb;")
+        if LANES == 1:
+            c.append("  if (jfe >= 16) {")
+            c.append("    #pragma unroll 4\n    for (int m_ = 0; m_ < 8; ++m_) {")
+            c.append("      const int si = ((2 * m_ + 1) * jfe) >> 4, j = jb0 + si * gS;")
+            c += ["      " + s for s in ev]
+            c += [f"      const bool ok = {fast};", "      " + up, "    }"]
+            c.append("    const int pc = pb, sp = jfe >> 5;")
+            c.append("    #pragma unroll 3\n    for (int m_ = 0; m_ < 6; ++m_) {")
+            c.append("      const int si_ = pc + (m_ < 3 ? m_ - 3 : m_ - 2) * sp;")
+            c.append("      const int si = min(max(si_, 0), jfe - 1), j = jb0 + si * gS;")
+            c += ["      " + s for s in ev]
+            c += [f"      const bool ok = {fast} && sp > 0 && si == si_;", "      " + up, "    }", "  }"]
+        else:
+            c.append(f"  if (jfe >= 32) for (int m_ = lane; m_ < 32; m_ += {LANES}) {{")
+            c.append("    const int si = ((2 * m_ + 1) * jfe) >> 6, j = jb0 + si * gS;")
+            c += ["    " + s for s in ev]
+            c += [f"    const bool ok = {fast};", "    " + up, "  }"]
+            c.append(f"  #pragma unroll\n  for (int w = {LANES} >> 1; w > 0; w >>= 1) {{")
+            c.append(f"    const {ST} b1 = __shfl_xor_sync(0xffffffffu, p1, w), b2 = __shfl_xor_sync(0xffffffffu, p2, w);")
+            c.append(f"    p2 = {fmax_}({fmin_}(p1, b1), {fmax_}(p2, b2)); p1 = {fmax_}(p1, b1);")
+            c.append("  }")
+        p_ = "p2" if fp32 else ("p1 - 1e-13 * (fabs(p1) + babs)" if verify else "p1")
+        c.append(f"  if (p1 > {ninf}) thr = {fmax_}(thr, {p_});")
+        c.append("}")
+        # group tests (NT at a time, branch-free, so that their chains overlap)
+        bv, bidx = ("v2", "idx2") if fp32 else ("v", "idx")
+        NT = self.LINE_TESTS
+        NB = max(1, min(self.LINE_BATCH, G // LANES))
+        cut = f"{fmax_}(thr, best[0].{bidx} >= 0 ? best[0].{bv} : {ninf})"
+        c += [f"const float th = {'' if fp32 else '__double2float_rd'}({cut});",
+              f"for (int g0 = 0; g0 * {G} < jfw; g0 += 32) {{",
+              "  unsigned need = 0u;",
+              f"  const int gc = min(32, (jfw + {G - 1}) / {G} - g0);",
+              f"  for (int b0 = lane; b0 < gc; b0 += {LANES * NT}) {{",
+              f"    float2 tm[{NT}]; float tu[{NT}]; int tl[{NT}], te[{NT}]; bool in_[{NT}];",
+              f"    #pragma unroll\n    for (int k = 0; k < {NT}; ++k) {{",
+              f"      const float4 gi = grp[min(g0 + b0 + {LANES} * k, gpc - 1)];",
+              "      const float t0 = gM * gi.y + gK, t1 = gM * gi.z + gK;",
+              "      const float lo = fminf(t0, t1) - gE, hi = fmaxf(t0, t1) + gE;",
+              "      const int L = (int)fminf(fmaxf(lo, 0.0f), gTop), H = min((int)fminf(fmaxf(hi, 0.0f), gTop) + 1, nA - 1);",
+              "      tu[k] = gi.x; tl[k] = L; te[k] = max(L, H - win + 1);",
+              "      in_[k] = lo >= 0.0f && hi <= gTop && te[k] - L <= (nlk - 1) * win;",
+              "      tm[k] = mrow[te[k]];",
+              "    }",
+              "    for (int q_ = 0; q_ < nlk - 1; ++q_) {  // uniform over the CTA",
+              f"      #pragma unroll\n      for (int k = 0; k < {NT}; ++k) {{",
+              "        const float2 v = mrow[min(tl[k] + q_ * win, te[k])];",
+              "        tm[k].x = lcm_nanmax(tm[k].x, v.x); tm[k].y = fmaxf(tm[k].y, v.y);",
+              "      }",
+              "    }",
+              f"    #pragma unroll\n    for (int k = 0; k < {NT}; ++k) {{",
+              f"      const int b_ = b0 + {LANES} * k;",
+              "      const bool skip = in_[k] && tu[k] + beta_b * tm[k].x + 4.8e-7f * (fabsf(tu[k]) + beta_b * tm[k].y) < th;",
+              f"      if (!skip && b_ < gc && (g0 + b_) * {G} < jfe) need |= 1u << b_;",
+              "    }",
+              "  }"]
+        if LANES > 1:
+            c.append(f"  #pragma unroll\n  for (int w = {LANES} >> 1; w > 0; w >>= 1) need |= __shfl_xor_sync(0xffffffffu, need, w);")
+        push = "push" if not multi else "put"
+        c += ["  unsigned any = __reduce_or_sync(0xffffffffu, need);",
+              "  while (any) {",
+              "    const int b_ = __ffs(any) - 1;",
+              "    any &= any - 1u;",
+              f"    const int i0 = (g0 + b_) * {G};",
+              f"    const int m = min({G}, gN - i0);",
+              "    if ((need >> b_) & 1u) {",
+              f"      for (int tb = lane; tb < m; tb += {LANES * NB}) {{",
+              f"        {ST} qv[{NB}], qm = {ninf}; unsigned okm = 0u; bool bad = false;",
+              f"        #pragma unroll\n        for (int k = 0; k < {NB}; ++k) {{",
+              f"          const int t = tb + {LANES} * k, j = jb0 + (i0 + min(t, m - 1)) * gS;"]
+        c += ["          " + s for s in ev]
+        c += [f"          const bool ok = {fast} && t < m;",
+              "          bad = bad || (ok && !lcm_isfinite(q));",
+              f"          qv[k] = ok ? q : {ninf};",
+              "          okm |= ok ? 1u << k : 0u;",
+              f"          qm = {fmax_}(qm, qv[k]);",
+              "        }"]
+        if verify:
+            c += [f"        const double cut = {cut};",
+                  "        if (okm && (bad || !(qm + 1e-13 * (fabs(qm) + babs) < cut))) {",
+                  f"          for (int k = 0; k < {NB}; ++k) {{",
+                  "            if (!((okm >> k) & 1u) || qv[k] + 1e-13 * (fabs(qv[k]) + babs) < cut) continue;",
+                  f"            const int j = jb0 + (i0 + tb + {LANES} * k) * gS;"]
+            c += ["            " + s for s in ev]
+            c += [f"            if ({call}) best[0].put(q, ad * n_ac + j);",
+                  "          }",
+                  "        }"]
+        else:
+            c += [f"        if (bad || (okm && (qm {'>=' if multi else '>'} best[0].{bv} || best[0].{bidx} < 0))) {{",
+                  f"          #pragma unroll\n          for (int k = 0; k < {NB}; ++k) {{",
+                  "            if (!((okm >> k) & 1u)) continue;",
+                  f"            const int j = jb0 + (i0 + tb + {LANES} * k) * gS;",
+                  f"            {ST} q = qv[k];",
+                  "            if (bad) {"]
+            c += ["              " + s for s in load("j")]
+            c += [f"              if (!{call}) continue;",
+                  "            }",
+                  f"            best[0].{push}(q, ad * n_ac + j);",
+                  "          }",
+                  "        }"]
+        c += ["      }",
+              "    }",
+              "  }",
+              "}"]
+        b += ["  " + s for s in c]
+        b.append("}")
+        o += ["  " + s for s in b]
+        o += ["}", "}"]
+        return o
 
     # ------------------------------------------------------------------ (d)
     def _sim_layout(self) -> None:

@@ -140,20 +140,44 @@ __device__ __forceinline__ T lcm_interp1(const S* __restrict__ row, int n, T c) 
   return lcm_zs(wl, v0) + lcm_zs(wu, v1);
 }
 
-// 1-D linear read of a float row in shared memory (the collapsed rows of the
-// single-precision search), with lcm_interp1's extrapolation and zero-safe
-// fallback.
-template <typename T>
-__device__ __forceinline__ T lcm_interp1s(const float* row, int n, T c) {
+// Fused and unfused combinations spelled out, so that a float search rounds
+// the same in every loop form.
+__device__ __forceinline__ float lcm_fma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ double lcm_fma(double a, double b, double c) { return __fma_rn(a, b, c); }
+__device__ __forceinline__ float lcm_lerp(float wl, float v0, float wu, float v1) {
+  return __fadd_rn(__fmul_rn(wl, v0), __fmul_rn(wu, v1));
+}
+__device__ __forceinline__ double lcm_lerp(double wl, double v0, double wu, double v1) {
+  return __dadd_rn(__dmul_rn(wl, v0), __dmul_rn(wu, v1));
+}
+
+// 1-D linear read of a row in shared memory (the collapsed rows of the
+// single-precision search, the rows of the line form), with lcm_interp1's
+// extrapolation and zero-safe fallback.
+template <typename T, typename S>
+__device__ __forceinline__ T lcm_interp1s(const S* row, int n, T c) {
   T lof;
   int lo = lcm_lower(c, n, lof);
   T wu = c - lof;
   T wl = T(1) - wu;
   T v0 = (T)row[lo];
   T v1 = (T)row[lo + 1];
-  T r = wl * v0 + wu * v1;
+  T r = lcm_lerp(wl, v0, wu, v1);
   if (lcm_isfinite(r)) return r;
   return lcm_zs(wl, v0) + lcm_zs(wu, v1);
+}
+
+// lcm_interp1s without the zero-safe rule, for callers that redo a result
+// that is not finite.
+template <typename T, typename S>
+__device__ __forceinline__ T lcm_interp1sf(const S* row, int n, T c) {
+  T lof;
+  int lo = lcm_lower(c, n, lof);
+  T wu = c - lof;
+  T wl = T(1) - wu;
+  T v0 = (T)row[lo];
+  T v1 = (T)row[lo + 1];
+  return lcm_lerp(wl, v0, wu, v1);
 }
 
 // 2-D bilinear read; `blk` is an (n0 x n1) row-major block.  Corner order and
@@ -184,6 +208,9 @@ __device__ __forceinline__ T lcm_interp2(const S* __restrict__ blk, int n0, int 
 __device__ __forceinline__ float lcm_nanmax(float a, float b) {
   return (a != a) ? a : ((b != b || b > a) ? b : a);
 }
+__device__ __forceinline__ double lcm_nanmax(double a, double b) {
+  return (a != a) ? a : ((b != b || b > a) ? b : a);
+}
 __device__ __forceinline__ float2 lcm_block16_stats(float x) {
   float mx = x, ab = lcm_isfinite(x) ? fabsf(x) : 0.0f;
 #pragma unroll
@@ -205,6 +232,11 @@ template <typename T> struct LcmBest {
   __device__ __forceinline__ void push(T q, int a) {
     if (q != q) { if (!nan) nan = a + 1; return; }
     if (idx < 0 || q > v) { v = q; idx = a; }
+  }
+  // an action in any order
+  __device__ __forceinline__ void put(T q, int a) {
+    if (q != q) { nan = nan ? min(nan, a + 1) : a + 1; return; }
+    if (idx < 0 || q > v || (q == v && a < idx)) { v = q; idx = a; }
   }
   // merge with another partial result over a disjoint action set; ties go to
   // the smaller flat index, so the result equals the sequential first argmax.
@@ -243,6 +275,11 @@ template <typename T> struct LcmBest2 {
       if (q > v || idx < 0) { v2 = v; idx2 = idx; v = q; idx = a; }
       else { v2 = q; idx2 = a; }
     }
+  }
+  // an action in any order (each at most once)
+  __device__ __forceinline__ void put(T q, int a) {
+    if (q != q) { nan = 1; return; }
+    if (q >= v2 || idx2 < 0) add(q, a);
   }
   __device__ __forceinline__ void merge(T ov, int oi, T ov2, int oi2, int onan) {
     nan |= onan;

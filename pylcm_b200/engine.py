@@ -164,6 +164,8 @@ class SolveEngine:
         self.device = device
         self.specs = model.regime_specs
         self._kernels: dict[tuple, RegimeKernels] = {}
+        self._bases: dict[tuple, RegimeKernels] = {}  # before the batch's launch shape is chosen
+        self._by_batch: dict[tuple, RegimeKernels] = {}  # (regime, targets, instances)
         self._traces: dict[tuple, TracedRegime] = {}
         self._targets: dict[tuple, tuple] = {}
 
@@ -183,17 +185,27 @@ class SolveEngine:
         return self.configs.get(spec.name) or default_config(spec, self.precision, n_items)
 
     def kernels(self, spec: RegimeSpec, targets: tuple[str, ...], params, n_items: int = 1) -> RegimeKernels:
+        rk = self._by_batch.get((spec.name, targets, n_items))
+        if rk is not None:
+            return rk
         cfg = self.config_for(spec, n_items)
+        base = self._bases.get((spec.name, targets, cfg))
+        if base is None:
+            tr = trace_regime(spec, self.specs, self.resolver(params), targets)
+            by = {s.name: s for s in self.specs}
+            base = RegimeKernels(tr, [by[t] for t in targets], self.precision, cfg)
+            self._bases[(spec.name, targets, cfg)] = base
+        if spec.name not in self.configs:
+            cfg = base.line_config(n_items)
         key = (spec.name, targets, cfg)
         rk = self._kernels.get(key)
         if rk is None:
-            tr = trace_regime(spec, self.specs, self.resolver(params), targets)
-            by = {s.name: s for s in self.specs}
-            rk = RegimeKernels(tr, [by[t] for t in targets], self.precision, cfg)
+            rk = base if cfg == base.cfg else RegimeKernels(base.tr, [t.spec for t in base.targets], self.precision, cfg)
             src = rk.source()
             rk.src = src
             rk.key = "lcm_" + hashlib.sha1(src.encode()).hexdigest()[:24]
             self._kernels[key] = rk
+        self._by_batch[(spec.name, targets, n_items)] = rk
         return rk
 
     def egm_kernels(self, spec: RegimeSpec, targets: tuple[str, ...], params):
@@ -565,9 +577,8 @@ class SolvePlan:
                     else:
                         r[base + 2] = self.sgrid[t.spec.name][pos].data_ptr()
             recs.append(r)
-        spt = rk.cfg.states_per_tile
         out["bell"] = np.stack(recs).astype(np.int64)
-        out["tiles"] = [math.ceil(s.n_states / spt)] * n
+        out["tiles"] = [rk.n_tiles()] * n
         out["atab_tiles"] = [math.ceil(s.n_actions / 256)] * n
         return out
 
