@@ -2713,7 +2713,8 @@ class RegimeKernels:
         # slot -- 0 the regime draw, 1 the taste shocks, then one per state
         # of each target (sim_slot)
         self.SW_JKEYS = w + 6
-        w += 7
+        self.SW_SPW = w + 7  # subjects per warp (1..32)
+        w += 8
         self.SW_ACT = w
         w += len(spec.actions)
         self.SW_SIN = w
@@ -2744,10 +2745,24 @@ class RegimeKernels:
     def _sim_kernel(self, env: dict) -> list[str]:
         """Kernel (d): one simulated period of this regime for every subject in it.
 
-        One warp per subject: the 32 lanes stride over the actions (double
-        precision), the first lane records value and action and draws the next
-        regime and next states with the Philox stream of (seed, subject,
-        period, stream id).  Stream ids: 0 regime draw, 1 + k the k-th state of
+        A warp takes up to 32 consecutive subjects (the item's subjects per
+        warp).  One subject after the other, its 32 lanes stride over the
+        actions (double precision), up to the longest prefix that can meet a
+        budget constraint on the slowest continuous action.  Then every lane
+        records value and action of its own subject and draws its next regime
+        and states, with the Philox stream of (seed, subject, period, stream
+        id): the draws do not depend on the subjects per warp.
+
+        What bounds it: issue and latency of the double-precision search; one
+        lane per warp drawing for its subject (a logarithm, square root and
+        cosine each) and the infeasible actions cost more than the feasible
+        ones.  B200, 16 x 10,000 subjects, 500 consumption points, 40 periods:
+        one subject per warp over every action 16.5 ms, 16 subjects per warp
+        over the feasible prefix 8.7, with the state phase per lane and the
+        warp reductions of lcm_warp_best 5.9 (32 / 8 / 4 subjects per warp:
+        7.0, 6.1, 7.4).
+
+        Stream ids: 0 regime draw, 1 + k the k-th state of
         the drawn target, 64 + d the taste shock of discrete choice d, 128 + k
         the mixture component of the k-th state (normal-mixture processes).
         """
@@ -2792,7 +2807,17 @@ class RegimeKernels:
 
         eS = Emitter("double", self.param_off, sim_prov("S"), "s")
         s_vals = [eS.emit(n) for n in bS]
-        eSD = Emitter("double", self.param_off, sim_prov("SD"), "x")
+        prov_sd = sim_prov("SD")
+        for a in spec.states:
+            # inside the search: the values of the subject at hand
+            if a.kind == "continuous":
+                prov_sd[id(ir.var("state", a.name, "f"))] = f"sv_{a.name}_b"
+            else:
+                prov_sd[id(ir.var("state", a.name, "i"))] = f"si_{a.name}_b"
+            if a.kind == "process":
+                node = ir.Expr("pidx", (proc_grid_name(a.name), ir.var("state", a.name, "i")), "f")
+                prov_sd[id(node)] = f"pv_{a.name}_b"
+        eSD = Emitter("double", self.param_off, prov_sd, "x")
         sdv = [eSD.emit(n) for n in bSD]
 
         ap(f"struct AFG_{tag} {{ const double* atf; const int* ati; int n; int a;")
@@ -2805,11 +2830,13 @@ class RegimeKernels:
         ap("  for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {")
         ap("    const int item = lcm_find_item(tile_prefix, n_items, tile);")
         ap(f"    const i64* __restrict__ it = items + (i64)item * {self.sim_words};")
-        ap("    const int s = (tile - tile_prefix[item]) * 8 + (int)threadIdx.x / 32;")
         ap("    const int lane = (int)threadIdx.x % 32;")
-        ap(f"    if (s >= lcm_wi(it, {self.SW_N})) continue;")
+        ap(f"    const int spw = lcm_wi(it, {self.SW_SPW});")
+        ap("    const int sub0 = ((tile - tile_prefix[item]) * 8 + (int)threadIdx.x / 32) * spw;")
         ap(f"    const int* rid_in = lcm_wp<const int>(it, {self.SW_RID_IN});")
-        ap(f"    if (rid_in[s] != {spec.rid}) continue;  // warp-uniform: one subject per warp")
+        ap(f"    const bool mine = lane < spw && sub0 + lane < lcm_wi(it, {self.SW_N}) && rid_in[sub0 + lane] == {spec.rid};")
+        ap("    unsigned todo = __ballot_sync(0xffffffffu, mine);")
+        ap("    if (todo == 0u) continue;  // warp-uniform")
         ap(f"    Ctx_{tag}<double, double> C; C.load(it);")
         ap(f"    const double* __restrict__ PV = lcm_wp<const double>(it, {self.W_P});")
         ap(f"    const int period = lcm_wi(it, {self.W_PERIOD});")
@@ -2819,16 +2846,16 @@ class RegimeKernels:
         ap(f"    const double* __restrict__ atf = lcm_wp<const double>(it, {self.W_ATAB});")
         ap(f"    const int* __restrict__ ati = reinterpret_cast<const int*>(atf + (i64){nf} * n_actions);")
         ap("    (void)period; (void)age; (void)ati; (void)PV;")
-        ap(f"    const u64 key = seed ^ (u64)it[{self.SW_SEED}];")
-        ap("    LcmRng rng; rng.k0 = (u32)key; rng.k1 = (u32)(key >> 32); rng.subject = (u32)s; rng.period = (u32)period;")
-        ap(f"    const u32* JK = lcm_wp<const u32>(it, {self.SW_JKEYS});")
-        ap("    const LcmJaxRng jr{JK, (u32)s};")
         for s_ in eP.lines:
             ap("    " + s_)
         ap(f"    double PVd[{nP}]; PVd[0] = 0.0;")
         for i, v in enumerate(pvals):
             ap(f"    PVd[{i}] = (double)({v});")
-        ap(f"    int SI[{NDS}]; int PLO[{NPROC}]; double PT[{NPROC}]; SI[0] = 0; PLO[0] = 0; PT[0] = 0.0;")
+
+        # every lane prepares its own subject (lanes without one repeat the
+        # warp's first), the search then reads the values by shuffles
+        ap("    const int s = sub0 + (mine ? lane : __ffs(todo) - 1);")
+        ap(f"    int SIo[{NDS}]; int PLOo[{NPROC}]; double PTo[{NPROC}]; SIo[0] = 0; PLOo[0] = 0; PTo[0] = 0.0;")
         for k, a in enumerate(spec.states):
             ap(f"    const double x_{a.name} = lcm_wp<const double>(it, {self.SW_SIN + k})[s];")
             if a.kind == "continuous":
@@ -2840,47 +2867,91 @@ class RegimeKernels:
                 pi = proc_names.index(a.name)
                 ap(f"    const double pv_{a.name} = x_{a.name};")
                 ap(f"    const double pc_{a.name} = lcm_coord_irreg<double>(pv_{a.name}, PV + {off}, {shape[0]});")
-                ap(f"    double pf_{a.name}; PLO[{pi}] = lcm_lower(pc_{a.name}, {shape[0]}, pf_{a.name}); PT[{pi}] = pc_{a.name} - pf_{a.name};")
-                ap(f"    const int si_{a.name} = PLO[{pi}];")
+                ap(f"    double pf_{a.name}; const int si_{a.name} = lcm_lower(pc_{a.name}, {shape[0]}, pf_{a.name});")
+                ap(f"    PLOo[{pi}] = si_{a.name}; PTo[{pi}] = pc_{a.name} - pf_{a.name};")
         for i, a in enumerate(dstates):
-            ap(f"    SI[{i}] = si_{a.name};")
+            ap(f"    SIo[{i}] = si_{a.name};")
         for s_ in eS.lines:
             ap("    " + s_)
-        ap(f"    double SV[{nS}]; SV[0] = 0.0;")
+        ap(f"    double SVo[{nS}]; SVo[0] = 0.0;")
         for i, v in enumerate(s_vals):
-            ap(f"    SV[{i}] = (double)({v});")
-        if taste:
-            ap(f"    LcmBest<double> bd[{ND}];")
-            ap(f"    #pragma unroll\n    for (int d = 0; d < {ND}; ++d) bd[d].init();")
+            ap(f"    SVo[{i}] = (double)({v});")
+        # the feasible prefix of the slowest continuous action
+        bb = self._budget_bound()
+        bexpr = None
+        if bb is not None:
+            kc, bnode = bb
+            if isinstance(bnode, (int, float)):
+                bexpr = repr(float(bnode))
+            for lst, fmt in ((bS, "SVo[{i}]"), (bP, "PVd[{i}]")):
+                for i, m in enumerate(lst):
+                    if m is bnode:
+                        bexpr = fmt.format(i=i)
+        if bexpr is None:
+            ap("    const int jfo = n_ac;")
         else:
-            ap("    LcmBest<double> best; best.init();")
-        ap(f"    #pragma unroll\n    for (int ad = 0; ad < {ND}; ++ad) {{")
+            ap(f"    const int ncg = lcm_wi(it, {self.W_ASIZE + kc});")
+            ap(f"    const int jfo = (lcm_row_bracket(lcm_wp<const double>(it, {self.W_AGRID + kc}), ncg, (double)({bexpr})) + 1)"
+               " * (n_ac / ncg);")
+        own = f"bo[{ND}]" if taste else "bo"
+        ap(f"    LcmBest<double> {own};  // of the lane's own subject")
+        ap("    while (todo) {")
+        ap("      const int src = __ffs(todo) - 1;")
+        ap("      todo &= todo - 1u;")
+        ap(f"      int SI[{NDS}]; int PLO[{NPROC}]; double PT[{NPROC}]; double SV[{nS}];")
+        for arr, n in (("SI", NDS), ("PLO", NPROC), ("PT", NPROC), ("SV", nS)):
+            ap(f"      #pragma unroll\n      for (int k = 0; k < {n}; ++k) {arr}[k] = __shfl_sync(0xffffffffu, {arr}o[k], src);")
+        ap("      const int jfe = __shfl_sync(0xffffffffu, jfo, src);")
+        if bSD:
+            # the state-and-choice phase reads the states
+            for a in spec.states:
+                if a.kind == "continuous":
+                    ap(f"      const double sv_{a.name}_b = __shfl_sync(0xffffffffu, sv_{a.name}, src);")
+                else:
+                    ap(f"      const int si_{a.name}_b = __shfl_sync(0xffffffffu, si_{a.name}, src);")
+                if a.kind == "process":
+                    ap(f"      const double pv_{a.name}_b = __shfl_sync(0xffffffffu, pv_{a.name}, src);")
+        if taste:
+            ap(f"      LcmBest<double> bd[{ND}];")
+            ap(f"      #pragma unroll\n      for (int d = 0; d < {ND}; ++d) bd[d].init();")
+        else:
+            ap("      LcmBest<double> best; best.init();")
+        ap(f"      #pragma unroll\n      for (int ad = 0; ad < {ND}; ++ad) {{")
         dl: list[str] = []
         decode_disc(dl, "ad")
         for s_ in dl + d_lines:
-            ap("      " + s_)
-        ap(f"      double DV[{nD}]; DV[0] = 0.0;")
+            ap("        " + s_)
+        ap(f"        double DV[{nD}]; DV[0] = 0.0;")
         for i, v in enumerate(d_vals):
-            ap(f"      DV[{i}] = (double)({v});")
+            ap(f"        DV[{i}] = (double)({v});")
         for s_ in eSD.lines:
-            ap("      " + s_)
-        ap(f"      double SDV[{nSD}]; SDV[0] = 0.0;")
+            ap("        " + s_)
+        ap(f"        double SDV[{nSD}]; SDV[0] = 0.0;")
         for i, v in enumerate(sdv):
-            ap(f"      SDV[{i}] = (double)({v});")
+            ap(f"        SDV[{i}] = (double)({v});")
         di_args = "".join(f"DI_{a.name}, " for a in dacts)
         push = "bd[ad].push(q, aidx);" if taste else "best.push(q, aidx);"
-        ap("      for (int j = lane; j < n_ac; j += 32) {")
-        ap("        const int aidx = ad * n_ac + j;")
-        ap(f"        AFG_{tag} af{{atf, ati, n_actions, aidx}};")
-        ap("        double q;")
-        ap(f"        if (lcm_simsa_{tag}<double, double>(C, PV, PVd, DV, SV, SDV, af, SI, PLO, PT, {di_args}period, age, q)) {push}")
+        ap("        for (int j = lane; j < jfe; j += 32) {")
+        ap("          const int aidx = ad * n_ac + j;")
+        ap(f"          AFG_{tag} af{{atf, ati, n_actions, aidx}};")
+        ap("          double q;")
+        ap(f"          if (lcm_simsa_{tag}<double, double>(C, PV, PVd, DV, SV, SDV, af, SI, PLO, PT, {di_args}period, age, q)) {push}")
+        ap("        }")
         ap("      }")
-        ap("    }")
         if taste:
-            ap(f"    #pragma unroll\n    for (int d = 0; d < {ND}; ++d) lcm_group_reduce<32, double>(bd[d]);")
+            ap(f"      #pragma unroll\n      for (int d = 0; d < {ND}; ++d) {{ lcm_warp_best(bd[d]); if (lane == src) bo[d] = bd[d]; }}")
         else:
-            ap("    lcm_group_reduce<32, double>(best);")
-        ap("    if (lane != 0) continue;")
+            ap("      lcm_warp_best(best);")
+            ap("      if (lane == src) bo = best;")
+        ap("    }")
+        ap("    if (!mine) continue;")
+        ap(f"    const u64 key = seed ^ (u64)it[{self.SW_SEED}];")
+        ap("    LcmRng rng; rng.k0 = (u32)key; rng.k1 = (u32)(key >> 32); rng.subject = (u32)s; rng.period = (u32)period;")
+        ap(f"    const u32* JK = lcm_wp<const u32>(it, {self.SW_JKEYS});")
+        ap("    const LcmJaxRng jr{JK, (u32)s};")
+        for a in spec.states:
+            if a.kind != "continuous":
+                ap(f"    (void)si_{a.name};")
         if taste:
             ap(f"    const double scale = lcm_wd(it, {self.W_TASTE});")
             # the reference (max_Q_over_a.py:268-297): per discrete cell the
@@ -2889,7 +2960,7 @@ class RegimeKernels:
             # the cells (a NaN cell first)
             ap("    int dstar = -1, dnan = -1; double bn = -lcm_lim<double>::inf(); double vstar = -lcm_lim<double>::inf();")
             ap(f"    for (int d = 0; d < {ND}; ++d) {{")
-            ap("      const double qc = bd[d].nan ? lcm_lim<double>::nan() : (bd[d].idx < 0 ? -lcm_lim<double>::inf() : bd[d].v);")
+            ap("      const double qc = bo[d].nan ? lcm_lim<double>::nan() : (bo[d].idx < 0 ? -lcm_lim<double>::inf() : bo[d].v);")
             ap("      const double g = JK ? jr.gumbel(1, d) : rng.gumbel(64u + (u32)d);")
             ap("      const double noisy = qc + scale * (g - 0.5772156649015329);")
             ap("      if (dnan < 0 && noisy != noisy) dnan = d;")
@@ -2898,13 +2969,13 @@ class RegimeKernels:
             ap("    if (dnan >= 0) { dstar = dnan; vstar = lcm_lim<double>::nan(); }")
             ap("    int aa = 0;")
             ap(f"    for (int d = 0; d < {ND}; ++d) if (d == dstar) "
-               "aa = bd[d].nan ? bd[d].nan - 1 : ((bd[d].idx < 0 || !(bd[d].v > -lcm_lim<double>::inf())) ? d * n_ac : bd[d].idx);")
+               "aa = bo[d].nan ? bo[d].nan - 1 : ((bo[d].idx < 0 || !(bo[d].v > -lcm_lim<double>::inf())) ? d * n_ac : bo[d].idx);")
             ap("    const double value = vstar;")
         else:
             # argmax_and_max (argmax.py:55-69): a NaN maximum matches no
             # entry, so the first action
-            ap("    const int aa = (best.nan || best.idx < 0) ? 0 : best.idx;")
-            ap("    const double value = best.nan ? lcm_lim<double>::nan() : (best.idx < 0 ? -lcm_lim<double>::inf() : best.v);")
+            ap("    const int aa = (bo.nan || bo.idx < 0) ? 0 : bo.idx;")
+            ap("    const double value = bo.nan ? lcm_lim<double>::nan() : (bo.idx < 0 ? -lcm_lim<double>::inf() : bo.v);")
         ap(f"    lcm_wp<double>(it, {self.SW_VAL})[s] = value;")
         ap(f"    lcm_wp<int>(it, {self.SW_AIDX})[s] = aa;")
         ap("    int arem = aa;")

@@ -314,6 +314,25 @@ __device__ __forceinline__ void lcm_group_reduce(LcmBest<T>& b) {
   }
 }
 
+// lcm_group_reduce<32, double> by warp reductions of the monotone 64-bit image
+// of the value (its halves in turn) and of the index: three reductions and a
+// broadcast instead of twenty shuffles.  Every lane gets the result.
+__device__ __forceinline__ void lcm_warp_best(LcmBest<double>& b) {
+  const unsigned full = 0xffffffffu;
+  if (__any_sync(full, b.nan != 0)) b.nan = (int)__reduce_min_sync(full, b.nan ? (u32)b.nan : 0x7fffffffu);
+  const u64 w = (u64)__double_as_longlong(b.v + 0.0);  // -0 ranks with 0
+  const u64 key = b.idx < 0 ? 0ull : ((w >> 63) ? ~w : (w | 0x8000000000000000ull));
+  const u32 hi = __reduce_max_sync(full, (u32)(key >> 32));
+  const bool top = b.idx >= 0 && (u32)(key >> 32) == hi;
+  const u32 lo = __reduce_max_sync(full, top ? (u32)key : 0u);
+  const bool first = top && (u32)key == lo;
+  const u32 idx = __reduce_min_sync(full, first ? (u32)b.idx : 0xffffffffu);
+  const unsigned own = __ballot_sync(full, first && (u32)b.idx == idx);
+  if (own == 0u) return;  // no feasible action on any lane
+  b.v = __shfl_sync(full, b.v, __ffs(own) - 1);
+  b.idx = (int)idx;
+}
+
 // Tile -> item lookup: prefix[i] is the first tile of item i, prefix[n] = total.
 __device__ __forceinline__ int lcm_find_item(const int* __restrict__ prefix, int n_items, int tile) {
   int lo = 0, hi = n_items - 1;

@@ -180,6 +180,17 @@ def jax_key_chain(model, params, seed: int) -> dict:
     return chain
 
 
+def subjects_per_warp(total: int) -> int:
+    """Subjects a warp of kernel (d) takes in turn: a power of two up to 32
+    that leaves the GPU (148 SMs, 16 resident warps each at the kernel's 128
+    registers) about four waves of warps, so that small simulations still fill
+    it and large ones draw for 32 subjects at once."""
+    spw = 1
+    while spw < 32 and 2 * spw * 4 * 148 * 16 <= total:
+        spw *= 2
+    return spw
+
+
 class SimPlan:
     """Device buffers and launches of the simulations of solve instances.
 
@@ -280,6 +291,7 @@ class SimPlan:
         # simulation words, built per (instance, regime, kernel) for all its
         # periods at once, then grouped per (period, kernel) with one sort
         by_kernel: dict[tuple, list] = {}
+        spw = subjects_per_warp(sum(b["N"] for b in self.inst))
         jtabs: list[np.ndarray] = []  # JAX-stream key tables, laid out in one device buffer
         jrefs: list[tuple] = []  # (rows array, row indices, table offsets in words)
         jwords = 0
@@ -291,7 +303,7 @@ class SimPlan:
             A0 = {n: t.data_ptr() for n, t in b["A"].items()}
             R0, V0, X0 = b["R"].data_ptr(), b["val"].data_ptr(), b["aidx"].data_ptr()
             seed_w = np.uint64(b["seed"]).astype(np.int64)
-            tiles = math.ceil(N / 8)
+            tiles = math.ceil(N / (8 * spw))
             pl, row = self.plan.instance_plan(b["idx"])
             for s in b["eng"].specs:
                 for rk, G, gp in pl.sim_groups().get(s.name, []):
@@ -308,6 +320,7 @@ class SimPlan:
                     rows[:, rk.SW_VAL] = V0 + pa * sbytes
                     rows[:, rk.SW_AIDX] = X0 + pa * ibytes
                     rows[:, rk.SW_SEED] = seed_w
+                    rows[:, rk.SW_SPW] = spw
                     for k, a in enumerate(s.actions):
                         rows[:, rk.SW_ACT + k] = A0[a.name] + pa * sbytes
                     for k, a in enumerate(s.states):
