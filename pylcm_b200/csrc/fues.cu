@@ -301,27 +301,48 @@ __global__ void __launch_bounds__(kBlock) fues_kernel(const double* __restrict__
 // ---------------------------------------------------------------------------
 // Shared-memory form (rows of up to kSmemMaxN candidates).
 //
-// Same three stages and the same decisions as fues_kernel, with the sorted
-// row staged in shared memory and the scan's per-step work cut to what a
-// step uses:
+// Same three stages and the same decisions as fues_kernel, with the row in
+// shared memory and the serial part cut to what it needs:
+//   * DC-EGM candidates arrive almost sorted (a value kink sends the
+//     endogenous grid back once; on the 2000-point retirement model 0 to 23
+//     descents in a row of 2020): an ascending row is not sorted at all, one
+//     of up to kMaxRuns ascending runs is merged by ranks (each candidate
+//     counts the smaller ones of every other run by binary search), and only
+//     a row of more runs goes through the bitonic network;
 //   * a step without a policy jump between j and i never reads the
-//     look-ahead, the intersections or i's own neighbours -- it is dropped
-//     or emits j and shifts (k, j) <- (j, i);
-//   * when j is the previous candidate (the common case), the policy-jump
-//     test and the secant of (j, i) are precomputed for every position in
-//     parallel before the scan; grad_before is the previous secant while k is
-//     the candidate before j, unmodified;
-//   * the look-ahead searches (warp ballot over shared memory) run only on
-//     steps with a policy jump.
-// Every value the scan uses is computed with the same operations and
-// operands as in fues_kernel, so the rows are identical.
+//     look-ahead, the intersections or i's own neighbours -- it is dropped or
+//     emits j and shifts (k, j) <- (j, i).  Whether that step is plain (keeps
+//     its candidate and only emits j) while j and k are the two candidates
+//     before it depends on the position alone: all threads put that bit in a
+//     mask, and the scan (warp 0) commits the run up to the next clear bit at
+//     once;
+//   * the policy-jump test divides only where a product with a rounding
+//     margin cannot decide it (policy_jump_fast);
+//   * the look-ahead searches run only on steps with a policy jump, 32
+//     candidates first, then 128 per step, and j's is kept while j stays;
+//   * candidates dropped one after the other are dropped 32 at a time;
+//   * the refined rows' NaN tail is filled after the scan, once.
+// Every decision is the one fues_kernel takes and every emitted value is
+// computed with the same operations and operands, so the rows are identical.
+//
+// What bounds it: the serial scan of the rows with many policy jumps (a few
+// rows of a launch; about 1.5 thousand cycles per jump, in dependent loads,
+// ballots and divisions) and the staging.  The row takes as little shared
+// memory as it can -- four doubles and an index per candidate, the sort keys
+// in the savings' place -- for three CTAs per SM at rows of 2020.  B200, 1056
+// rows of 2020 candidates per period (20 periods of the retirement model,
+// batch 32): 13.9 ms with a bitonic sort of every row and a step-by-step scan,
+// 7.4 ms in this form; with taste shocks (777 points, batch 12, 10 periods)
+// 1.76 and 0.57 ms.  Two CTAs per SM with 128 registers: 7.4 ms.  Searching
+// the neighbours of every jump ahead of the scan by all warps: slower (10 ms),
+// most of them are dropped without it.
 constexpr int kSmemMaxN = 4096;
 constexpr int kFuesItemWords = 13;
 
 __host__ __device__ constexpr size_t fues_smem_bytes(int n) {
   int np2 = 1;
   while (np2 < n) np2 <<= 1;
-  return (size_t)5 * n * sizeof(double) + (size_t)np2 * (sizeof(unsigned long long) + sizeof(int));
+  return (size_t)3 * n * sizeof(double) + (size_t)np2 * (sizeof(unsigned long long) + sizeof(unsigned short));
 }
 
 // Monotone 64-bit image of a grid value for the sort: NaN ranks with +inf and
@@ -413,69 +434,195 @@ struct FuesItems {
   }
 };
 
-// x[t] <- x[sidx[t]] for t < n, through the shared-memory buffer `tmp`
-__device__ __forceinline__ void permute_sorted(double* x, double* tmp, const int* sidx, int n) {
-  for (int t = threadIdx.x; t < n; t += kBlock) tmp[t] = x[sidx[t]];
+constexpr int kPerThread = kSmemMaxN / kBlock;  // candidates a thread holds in registers
+constexpr int kMaxRuns = 17;                    // ascending runs merged by ranks
+constexpr int kMaxSegments = 64;                // runs of plain steps copied by the whole CTA
+
+// x[t] <- x[sidx[t]] for t < n, through registers
+__device__ __forceinline__ void permute_sorted(double* x, const unsigned short* sidx, int n) {
+  double r[kPerThread];
+#pragma unroll
+  for (int k = 0; k < kPerThread; ++k) {
+    const int t = threadIdx.x + k * kBlock;
+    if (t < n) r[k] = x[sidx[t]];
+  }
   __syncthreads();
-  for (int t = threadIdx.x; t < n; t += kBlock) x[t] = tmp[t];
-  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < kPerThread; ++k) {
+    const int t = threadIdx.x + k * kBlock;
+    if (t < n) x[t] = r[k];
+  }
+}
+
+// policy_jump with the division only near the threshold: with t = thr |dx|
+// rounded once, |dy| beyond t (1 +- 1e-15) decides |dy / dx| > thr, however
+// the quotient rounds.
+__device__ __forceinline__ bool policy_jump_fast(double ga, double pa, double gb, double pb, double thr,
+                                                 bool use_sav, double sa, double sb) {
+  const double ia = ga - pa, ib = gb - pb;
+  if (ga == gb) return use_sav ? (sa != sb) : (ia != ib);
+  const double ad = fabs(ib - ia), t = thr * fabs(gb - ga);
+  if (t > 1e-290 && t < 1e300) {
+    if (ad > t * (1.0 + 1e-15)) return true;
+    if (ad < t * (1.0 - 1e-15)) return false;
+  }
+  return fabs(slope(ga, ia, gb, ib)) > thr;
+}
+
+// find_same_segment over shared memory: position of the nearest same-segment
+// candidate of (ag, ap) from idx in direction dir within `window` positions,
+// -1 if there is none (warp-cooperative; 32 candidates, then 128 at a time)
+__device__ __forceinline__ int find_same_segment_at(const double* g, const double* p, const double* v, int n,
+                                                    double ag, double ap, int idx, int dir, double thr, int window) {
+  const int lane = threadIdx.x & 31;
+  const int last = min(window, dir > 0 ? n - 1 - idx : idx);  // offsets 1 .. last
+  auto same = [&](int off) {
+    bool ok = false;
+    if (off <= last) {
+      const int k = idx + dir * off;
+      const double gk = g[k];
+      ok = !isnan_(gk) && !isnan_(v[k]) && !policy_jump_fast(ag, ap, gk, p[k], thr, false, 0.0, 0.0);
+    }
+    return ok;
+  };
+  if (last < 1) return -1;
+  unsigned m = __ballot_sync(0xffffffffu, same(1 + lane));
+  if (m) return idx + dir * __ffs(m);
+  for (int base = 33; base <= last; base += 128) {
+    unsigned b[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) b[q] = __ballot_sync(0xffffffffu, same(base + 32 * q + lane));
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+      if (b[q]) return idx + dir * (base + 32 * q + __ffs(b[q]) - 1);
+  }
+  return -1;
 }
 
 template <class Rows>
-__global__ void __launch_bounds__(kBlock) fues_smem_kernel(Rows rows) {
+__global__ void __launch_bounds__(kBlock, 3) fues_smem_kernel(Rows rows) {
   extern __shared__ __align__(16) unsigned char fues_smem[];
+  __shared__ unsigned plain_mask[kSmemMaxN / 32 + 1];
+  __shared__ int run_start[kMaxRuns];
+  __shared__ int3 segs[kMaxSegments];  // runs of plain steps to copy
+  __shared__ int n_desc, n_emit, n_runs;
   const int total = rows.count();
   const double nan = __longlong_as_double(0x7ff8000000000000LL);
+  const int tid = threadIdx.x, lane = tid & 31;
   for (int row = blockIdx.x; row < total; row += gridDim.x) {
     const FuesRowIO io = rows.row(row);
     const int n = io.n_in;
     const int n_out = io.n_out;
     const double thr = io.thr;
-    const double* G = io.G;
-    const double* P = io.P;
-    const double* V = io.V;
+    const double* __restrict__ G = io.G;
+    const double* __restrict__ P = io.P;
+    const double* __restrict__ V = io.V;
+    const double* __restrict__ S = io.S;
     int np2 = 1;
     while (np2 < n) np2 <<= 1;
+    // three arrays of n, then np2 words for the savings (the bitonic network's
+    // keys while it sorts), then the order
     double* g = reinterpret_cast<double*>(fues_smem);
     double* p = g + n;
     double* v = p + n;
     double* s = v + n;
-    double* sec = s + n;
-    unsigned long long* skey = reinterpret_cast<unsigned long long*>(sec + n);
-    int* sidx = reinterpret_cast<int*>(skey + np2);
+    unsigned long long* skey = reinterpret_cast<unsigned long long*>(s);
+    unsigned short* sidx = reinterpret_cast<unsigned short*>(skey + np2);
     __syncthreads();  // the previous row is done with shared memory
-    // ---- 1. stage the row in shared memory (input order), sort indices by
-    // the lexsort key read from there, then put each array in sorted order
-    // through registers
-    for (int t = threadIdx.x; t < n; t += kBlock) {
-      const double gt = G[t], pt = P[t];
-      g[t] = gt;
-      p[t] = pt;
-      v[t] = V[t];
-      s[t] = io.S ? io.S[t] : gt - pt;
+    // ---- 1. stage the row (input order), four candidates per thread in flight
+    if (tid == 0) n_desc = 0;
+    for (int t0 = tid; t0 < n; t0 += 4 * kBlock) {
+      double a[4], b[4], c[4], d[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int t = t0 + q * kBlock;
+        if (t < n) {
+          a[q] = __ldg(G + t);
+          b[q] = __ldg(P + t);
+          c[q] = __ldg(V + t);
+          d[q] = S ? __ldg(S + t) : 0.0;
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int t = t0 + q * kBlock;
+        if (t < n) {
+          g[t] = a[q];
+          p[t] = b[q];
+          v[t] = c[q];
+          s[t] = S ? d[q] : a[q] - b[q];
+        }
+      }
     }
     __syncthreads();
-    // (grid key, index) pairs: a compare-exchange reads positions t and
-    // t ^ stride; only equal grid keys consult value, policy and index
-    for (int t = threadIdx.x; t < np2; t += kBlock) {
-      sidx[t] = t;
-      skey[t] = t < n ? grid_key(g[t]) : ~0ULL;  // padding sorts last
+    // does position a's candidate come before position b's?
+    auto before = [&](int a, int b) { return !key_less(load_key(g, v, p, b, n), load_key(g, v, p, a, n)); };
+    for (int t = tid; t + 1 < n; t += kBlock) {
+      if (!before(t, t + 1)) {
+        const int q = atomicAdd(&n_desc, 1);
+        if (q < kMaxRuns - 1) run_start[q] = t + 1;
+      }
     }
     __syncthreads();
-    const int half = np2 >> 1;
-    for (int size = 2; size <= np2; size <<= 1) {
-      for (int stride = size >> 1; stride > 0; stride >>= 1) {
-        const int ls = __ffs(stride) - 1;  // stride = 2^ls
+    const int nd = n_desc;
+    if (nd > 0) {
+      for (int t = tid; t < np2; t += kBlock) skey[t] = t < n ? grid_key(g[t]) : ~0ULL;  // padding sorts last
+      __syncthreads();
+    }
+    if (nd > 0 && nd < kMaxRuns) {
+      // ranks: own place in the run plus, per other run, the candidates
+      // before this one
+      if (tid == 0) {
+        for (int a = 1; a < nd; ++a) {
+          const int x = run_start[a];
+          int b = a;
+          for (; b > 0 && run_start[b - 1] > x; --b) run_start[b] = run_start[b - 1];
+          run_start[b] = x;
+        }
+      }
+      __syncthreads();
+      for (int t = tid; t < n; t += kBlock) {
+        const unsigned long long key = skey[t];
+        int rank = 0, r0 = 0;
+        for (int r = 0; r <= nd; ++r) {
+          const int r1 = r < nd ? run_start[r] : n;
+          if (t >= r0 && t < r1) {
+            rank += t - r0;
+          } else {
+            int lo = r0, hi = r1;  // first of the run that does not come before t
+            while (lo < hi) {
+              const int mid = (lo + hi) >> 1;
+              const unsigned long long km = skey[mid];
+              if (km != key ? km < key : before(mid, t)) lo = mid + 1; else hi = mid;
+            }
+            rank += lo - r0;
+          }
+          r0 = r1;
+        }
+        sidx[rank] = (unsigned short)t;
+      }
+      __syncthreads();
+    } else if (nd >= kMaxRuns) {
+      // bitonic network over (key, index) pairs: a compare-exchange reads
+      // positions t and t ^ stride; only equal grid keys consult value,
+      // policy and index
+      for (int t = tid; t < np2; t += kBlock) {
+        sidx[t] = (unsigned short)t;
+      }
+      __syncthreads();
+      const int half = np2 >> 1;
+      for (int size = 2; size <= np2; size <<= 1) {
+        for (int stride = size >> 1; stride > 0; stride >>= 1) {
+          const int ls = __ffs(stride) - 1;  // stride = 2^ls
 #pragma unroll 4
-        for (int j = threadIdx.x; j < half; j += kBlock) {
-          // the j-th compare-exchange pair (t, t + stride) of this stage:
-          // the positions whose bit ls is clear, in order
-          const int t = ((j >> ls) << (ls + 1)) | (j & (stride - 1));
-          const int partner = t + stride;
-          {
+          for (int j = tid; j < half; j += kBlock) {
+            // the j-th compare-exchange pair (t, t + stride) of this stage:
+            // the positions whose bit ls is clear, in order
+            const int t = ((j >> ls) << (ls + 1)) | (j & (stride - 1));
+            const int partner = t + stride;
             const bool ascending = (t & size) == 0;
             const unsigned long long ka = skey[t], kb = skey[partner];
-            const int ia = sidx[t], ib = sidx[partner];
+            const unsigned short ia = sidx[t], ib = sidx[partner];
             bool a_first;  // does (ka, ia) come before (kb, ib)?
             if (ka != kb) {
               a_first = ka < kb;
@@ -489,16 +636,21 @@ __global__ void __launch_bounds__(kBlock) fues_smem_kernel(Rows rows) {
               sidx[partner] = ia;
             }
           }
+          __syncthreads();
         }
-        __syncthreads();
       }
     }
-    permute_sorted(g, sec, sidx, n);  // `sec` is free until the scan tables
-    permute_sorted(p, sec, sidx, n);
-    permute_sorted(v, sec, sidx, n);
-    permute_sorted(s, sec, sidx, n);
+    if (nd > 0) {
+      permute_sorted(g, sidx, n);
+      permute_sorted(p, sidx, n);
+      permute_sorted(v, sidx, n);
+      __syncthreads();  // the savings come back in place of the keys
+      for (int t = tid; t < n; t += kBlock) s[t] = S ? __ldg(S + sidx[t]) : g[t] - p[t];
+      __syncthreads();
+    }
     // ---- 2. coincident groups: keep the maximisers, one per savings source
-    for (int t = threadIdx.x; t < n; t += kBlock) {
+    unsigned drop_bits = 0u;  // bit k: the thread's k-th position goes
+    for (int k = 0, t = tid; t < n; ++k, t += kBlock) {
       const double gt = g[t];
       bool keep = !isnan_(gt);
       if (keep) {
@@ -507,38 +659,47 @@ __global__ void __launch_bounds__(kBlock) fues_smem_kernel(Rows rows) {
         while (hi + 1 < n && g[hi + 1] == gt) ++hi;
         if (hi > lo) {
           double vmax = -__longlong_as_double(0x7ff0000000000000LL);
-          for (int k = lo; k <= hi; ++k) {
-            const double vk = v[k];
-            if (!isnan_(vk) && vk > vmax) vmax = vk;
+          for (int q = lo; q <= hi; ++q) {
+            const double vq = v[q];
+            if (!isnan_(vq) && vq > vmax) vmax = vq;
           }
           keep = v[t] == vmax;
           if (keep) {
-            for (int k = lo; k < t; ++k)
-              if (v[k] == vmax && s[k] == s[t]) keep = false;
+            for (int q = lo; q < t; ++q)
+              if (v[q] == vmax && s[q] == s[t]) keep = false;
           }
         }
       }
-      sidx[t] = keep ? 1 : 0;
+      if (!keep) drop_bits |= 1u << k;
     }
     __syncthreads();
-    for (int t = threadIdx.x; t < n; t += kBlock) {
-      if (!sidx[t]) g[t] = p[t] = v[t] = s[t] = nan;
+    for (int k = 0, t = tid; t < n; ++k, t += kBlock) {
+      if ((drop_bits >> k) & 1u) g[t] = p[t] = v[t] = s[t] = nan;
     }
-    for (int t = threadIdx.x; t < n_out; t += kBlock) io.GO[t] = io.PO[t] = io.VO[t] = nan;
     __syncthreads();
-    // ---- 3a. per position t: policy jump and secant of (t - 1, t)
-    for (int t = threadIdx.x + 1; t < n; t += kBlock) {
-      sidx[t] = policy_jump(g[t - 1], p[t - 1], g[t], p[t], thr, true, s[t - 1], s[t]) ? 1 : 0;
-      sec[t] = slope(g[t - 1], v[t - 1], g[t], v[t]);
+    // ---- 3a. plain steps: while j and k are the two candidates before t, the
+    // step at t keeps candidate t and only emits j when t is valid, shows no
+    // policy jump from t - 1, and is neither below t - 1 nor a savings
+    // decrease with a secant under the previous one
+    for (int t = tid; t < ((n + 31) & ~31); t += kBlock) {
+      bool ok = false;
+      if (t >= 2 && t < n) {
+        const double gt = g[t], vt = v[t], g1 = g[t - 1], v1 = v[t - 1];
+        ok = !isnan_(gt) && !isnan_(vt) && !(vt < v1) &&
+             !policy_jump_fast(g1, p[t - 1], gt, p[t], thr, true, s[t - 1], s[t]);
+        if (ok && s[t] < s[t - 1]) ok = !(slope(g1, v1, gt, vt) < slope(g[t - 2], v[t - 2], g1, v1));
+      }
+      const unsigned m = __ballot_sync(0xffffffffu, ok);
+      if (lane == 0) plain_mask[t >> 5] = m;
     }
     __syncthreads();
     // ---- 3b. the scan (warp 0; all lanes hold the state, lane 0 writes)
-    if (threadIdx.x < 32) {
-      const int lane = threadIdx.x;
+    if (tid < 32) {
       double* GO = io.GO;
       double* PO = io.PO;
       double* VO = io.VO;
-      int cnt = 0;
+      const int words = (n + 31) >> 5;
+      int cnt = 0, n_seg = 0;
       auto emit = [&](double eg, double ep, double ev) {
         if (lane == 0 && cnt < n_out) {
           GO[cnt] = eg;
@@ -551,30 +712,43 @@ __global__ void __launch_bounds__(kBlock) fues_smem_kernel(Rows rows) {
       double gj = g[0], pj = p[0], vj = v[0], sj = s[0];
       int jidx = 0, kidx = 0;  // candidates j and k are (kidx < 0: k is a kink point)
       const double near = 16.0 * 2.220446049250313e-16;
+      const int span = io.window >= n ? 32 : 1;
+      int jn = -1;  // j's next same-segment candidate, while have_jn
+      bool have_jn = false;
       for (int idx = 1; idx < n; ++idx) {
-        // Runs of plain steps, 32 at a time.  While j and k are the two
-        // candidates before idx, step t keeps candidate t and only emits j
-        // when t is valid, shows no policy jump from t - 1, and is neither
-        // below t - 1 nor a savings decrease with a secant under the previous
-        // one -- all of it from the per-position tables.  Such a step leaves
-        // j = t - 1 + 1 and k = t - 1, so the next step's test is again a
-        // table lookup: the lanes test idx .. idx + 31 at once and the warp
-        // commits the leading run of passing steps (each emits its j).
-        if (kidx >= 0 && jidx == idx - 1 && kidx == jidx - 1) {
-          const int t = idx + lane;
-          bool ok = false;
-          if (t < n) {
-            const double gt = g[t], vt = v[t];
-            ok = !isnan_(gt) && !isnan_(vt) && sidx[t] == 0 && !(vt < v[t - 1]) &&
-                 !(s[t] < s[t - 1] && sec[t] < sec[t - 1]);
+        // the run of plain steps from idx ends at the next clear bit.  Its
+        // first step may follow any k if its savings do not decrease (the
+        // only test that reads k); the later ones follow t - 2 and t - 1
+        if (jidx == idx - 1 && ((kidx >= 0 && kidx == jidx - 1) || !(s[idx] < sj))) {
+          int stop = n;
+          for (int w0 = idx >> 5; w0 < words; w0 += 32) {
+            unsigned clear = 0u;
+            if (w0 + lane < words) {
+              clear = ~plain_mask[w0 + lane];
+              if (w0 + lane == idx >> 5) clear &= 0xffffffffu << (idx & 31);
+            }
+            const unsigned b = __ballot_sync(0xffffffffu, clear != 0u);
+            if (b) {
+              const int src = __ffs(b) - 1;
+              const unsigned c = __shfl_sync(0xffffffffu, clear, src);
+              stop = min(n, 32 * (w0 + src) + __ffs(c) - 1);
+              break;
+            }
           }
-          const unsigned fail = ~__ballot_sync(0xffffffffu, ok);
-          const int m = fail ? __ffs(fail) - 1 : 32;
+          const int m = stop - idx;
           if (m > 0) {
-            if (lane < m && cnt + lane < n_out) {
-              GO[cnt + lane] = g[idx - 1 + lane];
-              PO[cnt + lane] = p[idx - 1 + lane];
-              VO[cnt + lane] = v[idx - 1 + lane];
+            // its j's are copied by the whole CTA after the scan
+            if (n_seg < kMaxSegments) {
+              if (lane == 0) segs[n_seg] = make_int3(idx - 1, cnt, m);
+              ++n_seg;
+            } else {
+              for (int q = lane; q < m; q += 32) {
+                if (cnt + q < n_out) {
+                  GO[cnt + q] = g[idx - 1 + q];
+                  PO[cnt + q] = p[idx - 1 + q];
+                  VO[cnt + q] = v[idx - 1 + q];
+                }
+              }
             }
             cnt += m;
             const int nj = idx + m - 1;
@@ -582,61 +756,72 @@ __global__ void __launch_bounds__(kBlock) fues_smem_kernel(Rows rows) {
             kidx = nj - 1;
             gj = g[nj]; pj = p[nj]; vj = v[nj]; sj = s[nj];
             jidx = nj;
-            idx = nj;  // the loop's increment moves to the first untested step
+            have_jn = false;
+            idx = nj;  // the loop's increment moves to the first step not in the run
             continue;
           }
         }
-        const double gi = g[idx], vi = v[idx];
-        if (isnan_(gi) || isnan_(vi)) continue;
-        const double pi = p[idx], si = s[idx];
-        const bool prev = jidx == idx - 1;
-        const bool sw = prev ? (sidx[idx] != 0) : policy_jump(gj, pj, gi, pi, thr, true, sj, si);
-        const bool node_crossing = sw && gi == gj && vi == vj;
-        bool have_sec = false, have_gb = false;
-        double secant = 0.0, grad_before = 0.0;
-        auto get_secant = [&]() {
-          if (!have_sec) {
-            secant = prev ? sec[idx] : slope(gj, vj, gi, vi);
-            have_sec = true;
-          }
-          return secant;
-        };
-        auto get_gb = [&]() {
-          if (!have_gb) {
-            grad_before = (kidx >= 0 && kidx == jidx - 1) ? sec[jidx] : slope(gk, vk, gj, vj);
-            have_gb = true;
-          }
-          return grad_before;
-        };
-        bool drop = (vi < vj) && !sw;
-        if (!drop && si < sj) drop = get_secant() < get_gb();
-        double jg = nan, jp = nan, jv = nan;
-        bool jf = false;
-        if (sw) {
-          jf = find_same_segment(g, p, v, n, gj, pj, idx, 1, thr, io.window, jg, jp, jv);
-          if (!drop && jf) drop = (gi == jg) ? (vi < jv) : (get_secant() < slope(gi, vi, jg, jv));
+        // A dropped candidate leaves j and k as they are, so the lanes test
+        // idx .. idx + 31 against them at once and the warp drops the leading
+        // run.  j's next same-segment candidate jn is the same for every t
+        // before it (exhaustive look-ahead; a bounded one tests idx alone).
+        const int t = idx + lane;
+        const bool in = t < n && lane < span;
+        const double gt = in ? g[t] : nan, vt = in ? v[t] : nan, pt = in ? p[t] : nan, st = in ? s[t] : nan;
+        const bool valid = !isnan_(gt) && !isnan_(vt);
+        const bool jump = valid && policy_jump_fast(gj, pj, gt, pt, thr, true, sj, st);
+        const unsigned jumps = __ballot_sync(0xffffffffu, jump);
+        if (jumps && !(have_jn && (jn < 0 || jn > idx))) {
+          const bool same = valid && lane > 0 && (gt == gj ? (gj - pj == gt - pt) : !jump);
+          const unsigned ms = __ballot_sync(0xffffffffu, same);
+          jn = ms ? idx + __ffs(ms) - 1
+                  : find_same_segment_at(g, p, v, n, gj, pj, idx + span - 1, 1, thr, span == 1 ? io.window : n);
+          have_jn = span > 1;
         }
-        if (drop && !node_crossing) continue;
-        if (!sw) {
-          emit(gj, pj, vj);
-          gk = gj;
-          pk = pj;
-          vk = vj;
-          kidx = jidx;
-          gj = gi;
-          pj = pi;
-          vj = vi;
-          sj = si;
-          jidx = idx;
+        const bool jf = jumps != 0u && jn >= 0;
+        const double jg = jf ? g[jn] : nan, jp = jf ? p[jn] : nan, jv = jf ? v[jn] : nan;
+        bool drop = (vt < vj) && !jump;
+        if (valid && !drop && (st < sj || (jump && jf))) {
+          const double sec_t = slope(gj, vj, gt, vt);
+          if (st < sj) drop = sec_t < slope(gk, vk, gj, vj);
+          if (!drop && jump && jf) drop = (gt == jg) ? (vt < jv) : (sec_t < slope(gt, vt, jg, jv));
+        }
+        const bool open = jump && jf && t >= jn;  // needs the candidate after jn
+        const bool node = jump && gt == gj && vt == vj;
+        const unsigned stays = ~__ballot_sync(0xffffffffu, in && (!valid || (drop && !node && !open)));
+        const unsigned keeps = __ballot_sync(0xffffffffu, valid && !jump && !drop);
+        const int m = stays ? __ffs(stays) - 1 : 32;
+        const bool keep = m < 32 && ((keeps >> m) & 1u);
+        if (m > 0 || keep) {
+          idx += m;
+          if (keep) {  // the first one not dropped shows no jump: it only emits j
+            emit(gj, pj, vj);
+            gk = gj;
+            pk = pj;
+            vk = vj;
+            kidx = jidx;
+            gj = g[idx];
+            pj = p[idx];
+            vj = v[idx];
+            sj = s[idx];
+            jidx = idx;
+            have_jn = false;
+          } else {
+            --idx;
+          }
           continue;
         }
-        const double sc = get_secant();
-        const double gb = get_gb();
-        double fg, fp, fv, bg, bp, bv;
-        const bool ff = find_same_segment(g, p, v, n, gi, pi, idx, 1, thr, io.window, fg, fp, fv);
-        const bool bf = find_same_segment(g, p, v, n, gi, pi, idx, -1, thr, io.window, bg, bp, bv);
-        const bool found = ff || bf;
-        const double pg = ff ? fg : bg, pp = ff ? fp : bp, pv = ff ? fv : bv;
+        // a kept candidate across a policy jump
+        const double gi = g[idx], vi = v[idx], pi = p[idx], si = s[idx];
+        const bool node_crossing = gi == gj && vi == vj;
+        have_jn = false;  // j changes
+        const double sc = slope(gj, vj, gi, vi);
+        const double gb = slope(gk, vk, gj, vj);
+        // i's own neighbour: forward, or backward where there is none
+        int nb = find_same_segment_at(g, p, v, n, gi, pi, idx, 1, thr, io.window);
+        if (nb < 0) nb = find_same_segment_at(g, p, v, n, gi, pi, idx, -1, thr, io.window);
+        const bool found = nb >= 0;
+        const double pg = found ? g[nb] : nan, pp = found ? p[nb] : nan, pv = found ? v[nb] : nan;
         const double i_slope = slope(gi, vi, pg, pv);
         const double i_pslope = slope(gi, pi, pg, pp);
         const bool j_dom = found && (sc > i_slope) && !node_crossing;
@@ -689,8 +874,23 @@ __global__ void __launch_bounds__(kBlock) fues_smem_kernel(Rows rows) {
         jidx = idx;
       }
       if (!isnan_(gj) && !isnan_(vj)) emit(gj, pj, vj);
-      if (lane == 0) *io.nk = cnt;
+      if (lane == 0) {
+        *io.nk = cnt;
+        n_emit = cnt;
+        n_runs = n_seg;
+      }
     }
+    __syncthreads();
+    for (int r = 0; r < n_runs; ++r) {
+      const int3 seg = segs[r];  // (first position, first output, points)
+      const int m = min(seg.z, n_out - seg.y);
+      for (int q = tid; q < m; q += kBlock) {
+        io.GO[seg.y + q] = g[seg.x + q];
+        io.PO[seg.y + q] = p[seg.x + q];
+        io.VO[seg.y + q] = v[seg.x + q];
+      }
+    }
+    for (int t = n_emit + tid; t < n_out; t += kBlock) io.GO[t] = io.PO[t] = io.VO[t] = nan;
   }
 }
 
