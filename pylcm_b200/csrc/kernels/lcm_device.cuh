@@ -571,6 +571,49 @@ __device__ __forceinline__ int lcm_row_bracket(const double* __restrict__ xp, in
   return lo - 1;
 }
 
+// The limited end slopes (Fritsch & Carlson) of the cubic on a bracket, as
+// lcm_bracket_read uses them: they depend on the bracket alone, so a carry row
+// keeps them beside its nodes.  LCM_LINEAR in e0 marks a bracket read linearly
+// (a node value or slope that is not finite, or no width).
+#define LCM_LINEAR_BITS 0x7ffa5a5a5a5a5a5aLL
+__device__ __forceinline__ void lcm_bracket_slopes(double x0, double x1, double f0, double f1, double d0, double d1,
+                                                   double& e0, double& e1) {
+  const double h = x1 - x0;
+  if (lcm_isfinite(f0) && lcm_isfinite(f1) && lcm_isfinite(d0) && lcm_isfinite(d1) && h > 0.0) {
+    const double delta = (f1 - f0) / h;
+    e0 = e1 = 0.0;
+    if (delta != 0.0) {
+      double a = d0 / delta, bb = d1 / delta;
+      a = a > 0.0 ? a : 0.0;
+      bb = bb > 0.0 ? bb : 0.0;
+      const double r2 = a * a + bb * bb;
+      const double tau = r2 > 9.0 ? 3.0 / sqrt(r2) : 1.0;
+      e0 = tau * a * delta;
+      e1 = tau * bb * delta;
+    }
+  } else {
+    e0 = __longlong_as_double(LCM_LINEAR_BITS);
+    e1 = 0.0;
+  }
+}
+
+// lcm_bracket_read of a carried row with slopes, its end slopes known.
+__device__ __forceinline__ void lcm_bracket_read_known(double x0, double x1, double f0, double f1, double d0, double d1,
+                                                       double e0, double e1, int idx, double xq, double& val,
+                                                       double& slope_val) {
+  const double h = x1 - x0;
+  const double t = h > 0.0 ? (xq - x0) / h : 0.0;
+  double v = h > 0.0 ? f0 + t * (f1 - f0) : f1;
+  slope_val = h > 0.0 ? d0 + t * (d1 - d0) : d1;
+  if (__double_as_longlong(e0) != LCM_LINEAR_BITS && idx >= 0) {
+    const double t2 = t * t, t3 = t2 * t;
+    v = (2 * t3 - 3 * t2 + 1) * f0 + (t3 - 2 * t2 + t) * h * e0 + (-2 * t3 + 3 * t2) * f1 + (t3 - t2) * h * e1;
+  }
+  const bool neg0 = f0 == -LCM_INF, neg1 = f1 == -LCM_INF;
+  if (idx >= 0 && (neg0 || neg1) && !((xq == x0) && lcm_isfinite(f0)) && !((xq == x1) && lcm_isfinite(f1))) v = -LCM_INF;
+  val = v;
+}
+
 // The read on one bracket [x0, x1] (node values f0, f1, node slopes d0, d1
 // when has_dp) of a row whose bracket index is idx (-1: below the first node;
 // the bracket is then the first one) and idx <= L - 2.
@@ -604,14 +647,6 @@ __device__ __forceinline__ void lcm_bracket_read(double x0, double x1, double f0
   slope_val = s;
 }
 
-// lcm_row_bracket for the 32 converged lanes of a warp reading the same
-// sorted row (same xp and L on every lane; `xq` per lane): the brackets of
-// the warp's smallest and largest query bound every lane's bracket, so when
-// at most 32 nodes lie between them each lane counts the nodes at or below
-// its query among those (held one per lane, searched through shuffles)
-// instead of searching the row in memory.  The result equals
-// lcm_row_bracket's on every lane (a NaN query gets L - 1, as there); with a
-// wider window every lane falls back to its own search.
 // lcm_row_bracket of two warp-uniform queries qa, qb (same xp and L on every
 // lane of a converged warp) by a 32-ary search: each round every lane tests
 // one node of the current interval and a ballot keeps the sub-interval that
@@ -653,45 +688,12 @@ __device__ __forceinline__ void lcm_row_bracket_coop2(const double* __restrict__
   ib = blo - 1;
 }
 
-__device__ __forceinline__ int lcm_row_bracket_warp(const double* __restrict__ xp, int L, double xq) {
-  const unsigned full = 0xffffffffu;
-  double qmin = xq, qmax = xq;  // fmin / fmax skip NaN queries
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    qmin = fmin(qmin, __shfl_xor_sync(full, qmin, o));
-    qmax = fmax(qmax, __shfl_xor_sync(full, qmax, o));
-  }
-  if (qmin != qmin) return L - 1;  // every query is NaN
-  int i_lo, i_hi;
-  lcm_row_bracket_coop2(xp, L, qmin, qmax, i_lo, i_hi);
-  const int W = i_hi - i_lo;  // nodes in (i_lo, i_hi]
-  if (W > 32) {
-    // every lane's first node above its query lies in [i_lo + 1, i_hi + 1]
-    if (xq != xq) return L - 1;
-    int lo = i_lo + 1, hi = i_hi + 1;
-    while (lo < hi) { const int mid = (lo + hi) >> 1; if (xp[mid] > xq) hi = mid; else lo = mid + 1; }
-    return lo - 1;
-  }
-  const int lane = threadIdx.x & 31;
-  const double node = lane < W ? xp[i_lo + 1 + lane] : LCM_INF;
-  int lo = 0, hi = W;
-#pragma unroll
-  for (int s = 0; s < 6; ++s) {
-    const int mid = (lo + hi) >> 1;
-    const double x = __shfl_sync(full, node, mid & 31);
-    if (lo < hi) {
-      if (x > xq) hi = mid; else lo = mid + 1;
-    }
-  }
-  return xq != xq ? L - 1 : i_lo + lo;
-}
-
 __device__ __forceinline__ void lcm_row_read(const double* __restrict__ xp, const double* __restrict__ fp,
                                              const double* __restrict__ dp, int L, double xq,
-                                             double& val, double& slope_val, bool warp_uniform = false) {
+                                             double& val, double& slope_val) {
   if (L <= 0) { val = slope_val = LCM_NAN; return; }
   if (L == 1) { val = fp[0]; slope_val = dp ? dp[0] : LCM_NAN; return; }
-  const int idx = warp_uniform ? lcm_row_bracket_warp(xp, L, xq) : lcm_row_bracket(xp, L, xq);
+  const int idx = lcm_row_bracket(xp, L, xq);
   if (idx >= L - 1) { val = fp[L - 1]; slope_val = dp ? dp[L - 1] : LCM_NAN; return; }
   const int b = idx < 0 ? 0 : idx;
   lcm_bracket_read(xp[b], xp[b + 1], fp[b], fp[b + 1], dp ? dp[b] : 0.0, dp ? dp[b + 1] : 0.0, dp != nullptr, idx, xq,
@@ -699,99 +701,81 @@ __device__ __forceinline__ void lcm_row_read(const double* __restrict__ xp, cons
 }
 
 // lcm_row_read of K rows at the same per-lane query, for the 32 converged
-// lanes of a warp that read the same K rows (row k: xp[k], fp[k], dp[k], L[k]
-// equal on every lane).  The rows' searches run interleaved -- one 32-ary
-// ballot search with 2K heads (each row's bracket of the warp's smallest and
-// largest query), then each row's window search -- so their dependent loads
-// overlap.  Every result equals lcm_row_read's.
+// lanes of a warp that read the same K rows (row k: xp[k], fp[k], dp[k], its
+// brackets' end slopes ep[k], L[k] equal on every lane).  [qmin, qmax] is the range of the warp's queries
+// (fmin / fmax: NaN queries aside; NaN when every query is).
+//
+// A warp's queries of neighbouring savings nodes fall on some 30 to 40
+// consecutive nodes of a row, at about the same position in the rows of the
+// target's other discrete states.  The warp loads 64 nodes from `hint[k]`
+// (where the row read before had them, moved a little to the left), checks
+// that they cover the range, puts them in shared memory (`win`, one set per
+// warp) and every lane finds its bracket there in six steps.  Where they do
+// not cover it, a 32-ary search of the row places the window; a range wider
+// than the window falls back to a search per lane.  Every result equals
+// lcm_row_read's.
 template <int K>
-__device__ __forceinline__ void lcm_row_read_warpk(const double* const* xp, const double* const* fp,
-                                                   const double* const* dp, const int* L, double xq, double* val,
-                                                   double* slope_val) {
+__device__ __forceinline__ void lcm_row_read_win(const double* const* xp, const double* const* fp,
+                                                 const double* const* dp, const double2* const* ep, const int* L,
+                                                 double xq, double qmin, double qmax, int* hint, double (*win)[64],
+                                                 double* val, double* slope_val) {
   const unsigned full = 0xffffffffu;
   const int lane = threadIdx.x & 31;
-  double qmin = xq, qmax = xq;  // fmin / fmax skip NaN queries
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    qmin = fmin(qmin, __shfl_xor_sync(full, qmin, o));
-    qmax = fmax(qmax, __shfl_xor_sync(full, qmax, o));
-  }
   const bool all_nan = qmin != qmin;
-  // heads 2k, 2k + 1: row k at qmin, qmax (rows of fewer than 2 nodes, or
-  // every query NaN: no search)
-  int lo[2 * K], hi[2 * K];
-#pragma unroll
-  for (int h = 0; h < 2 * K; ++h) {
-    lo[h] = 0;
-    hi[h] = (L[h >> 1] >= 2 && !all_nan) ? L[h >> 1] : 0;
-  }
-  bool active = true;
-  while (active) {
-    bool up[2 * K];
-    int s[2 * K];
-#pragma unroll
-    for (int h = 0; h < 2 * K; ++h) {
-      s[h] = (hi[h] - lo[h] + 31) >> 5;
-      const int m = lo[h] + (lane + 1) * s[h] - 1;
-      const double q = (h & 1) ? qmax : qmin;
-      up[h] = lo[h] < hi[h] && (m >= hi[h] || xp[h >> 1][m] > q);
-    }
-    active = false;
-#pragma unroll
-    for (int h = 0; h < 2 * K; ++h) {
-      const unsigned b = __ballot_sync(full, up[h]);
-      if (lo[h] < hi[h]) {
-        if (b == 0u) {
-          lo[h] = hi[h];
-        } else {
-          const int f = __ffs(b) - 1, mf = lo[h] + (f + 1) * s[h] - 1;
-          lo[h] += f * s[h];
-          hi[h] = mf < hi[h] ? mf : hi[h];
-        }
-      }
-      active = active || lo[h] < hi[h];
-    }
-  }
-  // each row's window (i_lo, i_hi]: one node per lane, then a shuffle search
-  double node[K];
+  int ws[K];
+  bool wide[K];
+  double n0[K], n1[K];
 #pragma unroll
   for (int k = 0; k < K; ++k) {
-    const int i_lo = lo[2 * k] - 1, W = lo[2 * k + 1] - lo[2 * k];
-    node[k] = (L[k] >= 2 && !all_nan && W <= 32 && lane < W) ? xp[k][i_lo + 1 + lane] : LCM_INF;
+    ws[k] = max(0, min(hint[k], L[k] - 64));
+    n0[k] = ws[k] + lane < L[k] ? __ldg(xp[k] + ws[k] + lane) : LCM_INF;
+    n1[k] = ws[k] + 32 + lane < L[k] ? __ldg(xp[k] + ws[k] + 32 + lane) : LCM_INF;
   }
-  int idx[K];
 #pragma unroll
   for (int k = 0; k < K; ++k) {
-    const int i_lo = lo[2 * k] - 1, W = lo[2 * k + 1] - lo[2 * k];
-    int a = 0, z = W;
+    auto covers = [&]() {
+      const double a = __shfl_sync(full, n0[k], 0), z = __shfl_sync(full, n1[k], 31);
+      return (ws[k] == 0 || a <= qmin) && (ws[k] + 64 >= L[k] || z > qmax);
+    };
+    wide[k] = false;
+    if (!all_nan && !covers()) {  // warp-uniform
+      int ia, ib;
+      lcm_row_bracket_coop2(xp[k], L[k], qmin, qmax, ia, ib);
+      ws[k] = max(0, min(ia, L[k] - 64));
+      n0[k] = ws[k] + lane < L[k] ? __ldg(xp[k] + ws[k] + lane) : LCM_INF;
+      n1[k] = ws[k] + 32 + lane < L[k] ? __ldg(xp[k] + ws[k] + 32 + lane) : LCM_INF;
+      wide[k] = !covers();
+    }
+    // the next row's window starts a little left of this one's first bracket
+    hint[k] = ws[k] + __popc(__ballot_sync(full, n0[k] <= qmin)) + __popc(__ballot_sync(full, n1[k] <= qmin)) - 9;
+  }
+  __syncwarp();  // the lanes' reads of the last window are done
 #pragma unroll
-    for (int st = 0; st < 6; ++st) {
-      const int mid = (a + z) >> 1;
-      const double x = __shfl_sync(full, node[k], mid & 31);
-      if (a < z && W <= 32) {
-        if (x > xq) z = mid; else a = mid + 1;
-      }
-    }
-    if (W > 32 && xq == xq) {
-      // every lane's first node above its query lies in [i_lo + 1, i_hi + 1]
-      a = i_lo + 1;
-      z = lo[2 * k + 1];
-      while (a < z) { const int mid = (a + z) >> 1; if (xp[k][mid] > xq) z = mid; else a = mid + 1; }
-      idx[k] = a - 1;
-    } else {
-      idx[k] = (xq != xq || all_nan) ? L[k] - 1 : i_lo + a;
-    }
+  for (int k = 0; k < K; ++k) {
+    win[k][lane] = n0[k];
+    win[k][32 + lane] = n1[k];
+  }
+  __syncwarp();
+  int pos[K];  // nodes of the window at or below the query
+#pragma unroll
+  for (int k = 0; k < K; ++k) pos[k] = 0;
+#pragma unroll
+  for (int st = 32; st > 0; st >>= 1) {
+#pragma unroll
+    for (int k = 0; k < K; ++k) pos[k] += win[k][pos[k] + st - 1] <= xq ? st : 0;
   }
 #pragma unroll
   for (int k = 0; k < K; ++k) {
     const int Lk = L[k];
+    int ix = ws[k] + pos[k] + (win[k][pos[k]] <= xq ? 1 : 0) - 1;
+    if (wide[k]) ix = lcm_row_bracket(xp[k], Lk, xq);
+    if (xq != xq) ix = Lk - 1;
     if (Lk <= 0) { val[k] = slope_val[k] = LCM_NAN; continue; }
-    if (Lk == 1) { val[k] = fp[k][0]; slope_val[k] = dp[k] ? dp[k][0] : LCM_NAN; continue; }
-    const int ix = idx[k];
-    if (ix >= Lk - 1) { val[k] = fp[k][Lk - 1]; slope_val[k] = dp[k] ? dp[k][Lk - 1] : LCM_NAN; continue; }
+    if (Lk == 1) { val[k] = fp[k][0]; slope_val[k] = dp[k][0]; continue; }
+    if (ix >= Lk - 1) { val[k] = fp[k][Lk - 1]; slope_val[k] = dp[k][Lk - 1]; continue; }
     const int b = ix < 0 ? 0 : ix;
-    const double* d = dp[k];
-    lcm_bracket_read(xp[k][b], xp[k][b + 1], fp[k][b], fp[k][b + 1], d ? d[b] : 0.0, d ? d[b + 1] : 0.0, d != nullptr,
-                     ix, xq, val[k], slope_val[k]);
+    const double2 e = __ldg(ep[k] + b);
+    lcm_bracket_read_known(__ldg(xp[k] + b), __ldg(xp[k] + b + 1), __ldg(fp[k] + b), __ldg(fp[k] + b + 1),
+                           __ldg(dp[k] + b), __ldg(dp[k] + b + 1), e.x, e.y, ix, xq, val[k], slope_val[k]);
   }
 }

@@ -64,6 +64,8 @@ class EgmKernels:
         self.W_CM = take() if self.er.envelope == "rfc" else -1
         self.W_EV0 = take()
         self.W_RG, self.W_RC, self.W_RV, self.W_MU, self.W_NK = take(), take(), take(), take(), take()
+        # the refined rows' bracket end slopes (pairs), read by the continuation
+        self.W_ES = take()
         self.W_V = take()
         self.W_POL = take()
         self.W_NPAD = take()
@@ -77,7 +79,8 @@ class EgmKernels:
             elif t.is_value:
                 self.W_T.append({"tv": take(), "tm": take(), "tg": take(), "tn": take()})
             else:
-                self.W_T.append({"rg": take(), "rv": take(), "mu": take(), "nk": take(), "npad": take(), "taste": take()})
+                self.W_T.append({"rg": take(), "rv": take(), "mu": take(), "nk": take(), "npad": take(), "taste": take(),
+                                 "es": take()})
         self.n_words = w
 
     def names(self) -> tuple[str, str, str]:
@@ -192,17 +195,26 @@ class EgmKernels:
         base_prov = {id(ir.var("period", "period", "i")): "period", id(ir.var("age", "age", "f")): "age"}
 
         # ------------------------------------------------------------ (c1)
-        # latency-bound (dependent binary-search loads): at least 3 CTAs per
-        # SM (<= 85 registers) -- measured 26 % faster than the compiler's
-        # 88-register, 2-CTA choice on the 2000-node DC-EGM model
+        # bound by the latency of dependent loads and by issue (16 shocks x 2
+        # choices per candidate, a bracket search and a cubic each): at least
+        # 3 CTAs per SM (<= 85 registers) -- measured 26 % faster than the
+        # compiler's 88-register, 2-CTA choice on the 2000-node DC-EGM model.
+        # B200, batch 32, 2000 savings nodes: 1.04 ms per launch with a 32-ary
+        # search of every row and the limited slopes computed per read (1250
+        # instructions per warp and row pair), 0.76 with node windows placed
+        # by the row before (lcm_row_read_win), 0.61 with the end slopes kept
+        # beside the rows (560 instructions; the carry kernel that writes them
+        # 70 -> 108 us)
         ap(f'extern "C" __global__ void __launch_bounds__(256, 3) {cname}(const i64* __restrict__ items, '
            "const int* __restrict__ tile_prefix, int n_items, int n_tiles) {")
+        ap("  __shared__ double read_win[8][2][64];  // node windows of each warp's row reads")
+        ap("  double (*win)[64] = read_win[threadIdx.x / 32];")
         ap("  for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {")
         ap("    const int item = lcm_find_item(tile_prefix, n_items, tile);")
         ap(f"    const i64* __restrict__ it = items + (i64)item * {self.n_words};")
         ap(f"    const double* __restrict__ PV = lcm_wp<const double>(it, {self.W_P});")
         ap(f"    const int period = lcm_wi(it, {self.W_PERIOD}); const double age = lcm_wd(it, {self.W_AGE});")
-        ap("    (void)period; (void)age;")
+        ap("    (void)period; (void)age; (void)win;")
         ap(f"    const int n_sav = lcm_wi(it, {self.W_NSAV});")
         ap(f"    const int nc = {er.n_constrained};")
         ap("    const int n_cand = nc + n_sav;")
@@ -213,7 +225,7 @@ class EgmKernels:
         ap(f"    const int e = live ? e_t : {nrow} * n_sav - 1;")
         ap("    const int row = e / n_sav, j = e % n_sav;")
         # one candidate row for the whole warp: its carry-row reads share
-        # their bracket search (lcm_row_bracket_warp)
+        # their bracket search (lcm_row_read_win)
         # (the shuffle runs on every lane: a shuffle inside the short-circuit
         # of `live && ...` would leave the warp's non-live lanes out of it)
         ap("    const int row_l0 = __shfl_sync(0xffffffffu, row, 0);")
@@ -274,8 +286,23 @@ class EgmKernels:
                 body.append(f"    const double* RV = lcm_wp<const double>(it, {w['rv']});")
                 body.append(f"    const double* RM = lcm_wp<const double>(it, {w['mu']});")
                 body.append(f"    const int* NK = lcm_wp<const int>(it, {w['nk']});")
+                body.append(f"    const double2* ES = lcm_wp<const double2>(it, {w['es']}); (void)ES;")
                 body.append(f"    const int npad = lcm_wi(it, {w['npad']}); const double lam = lcm_wd(it, {w['taste']});")
                 body.append("    double nv = 0.0, nm = 0.0, den = 0.0;")
+                # the shared search needs the row's control flow to be the
+                # same on every lane: the regime probability and the node
+                # weights must not depend on the savings node
+                uniform = not any(n is A_VAR for n in ir.topo_order([ir.const(x) for x in self._row_exprs(t)]))
+                if uniform:
+                    body.append("    double qmin = Rn, qmax = Rn;  // the warp's queries (fmin / fmax skip NaN)")
+                    body.append("    if (warp_row) {")
+                    body.append("      #pragma unroll\n      for (int o = 16; o > 0; o >>= 1) {")
+                    body.append("        qmin = fmin(qmin, __shfl_xor_sync(0xffffffffu, qmin, o));")
+                    body.append("        qmax = fmax(qmax, __shfl_xor_sync(0xffffffffu, qmax, o));")
+                    body.append("      }")
+                    body.append("    }")
+                    body.append(f"    int hint[{nd_t}];")
+                    body.append(f"    #pragma unroll\n    for (int d = 0; d < {nd_t}; ++d) hint[d] = 0;")
                 body.append(f"    for (int jc = 0; jc < {J}; ++jc) {{")
                 body.append("      int jr = jc; double wt = 1.0;")
                 for ax, arr in reversed(wl_names):
@@ -283,41 +310,31 @@ class EgmKernels:
                 body.append("      den += wt;")
                 body.append("      if (wt == 0.0) continue;")
                 body.append(f"      double vals[{nd_t}], mus[{nd_t}];")
-                # the shared search needs the row's control flow to be the
-                # same on every lane: the regime probability and the node
-                # weights must not depend on the savings node
-                uniform = not any(n is A_VAR for n in ir.topo_order([ir.const(x) for x in self._row_exprs(t)]))
-                flag = "warp_row" if uniform else "false"
                 single = [f"      for (int d = 0; d < {nd_t}; ++d) {{",
                           f"        const i64 crow = (i64)jc * {nd_t} + d;",
                           "        const int Lk = min(NK[crow], npad);",
                           "        lcm_row_read(RG + crow * npad, RV + crow * npad, RM + crow * npad, "
-                          f"NK[crow] > npad ? 0 : Lk, Rn, vals[d], mus[d], {{flag}});",
+                          "NK[crow] > npad ? 0 : Lk, Rn, vals[d], mus[d]);",
                           "      }"]
-                if uniform and nd_t >= 2:
+                if uniform:
                     # a warp reading one candidate row reads the choices'
                     # child rows in pairs, their searches interleaved
                     body.append("      if (warp_row) {")
-                    for d0 in range(0, nd_t - 1, 2):
+                    for d0 in range(0, nd_t, 2):
+                        K = min(2, nd_t - d0)
                         body.append("        {")
-                        body.append("          const double* xs[2]; const double* fs[2]; const double* ds[2]; int Ls[2];")
-                        for k in range(2):
+                        body.append(f"          const double* xs[{K}]; const double* fs[{K}]; const double* ds[{K}]; const double2* es[{K}]; int Ls[{K}];")
+                        for k in range(K):
                             body.append(f"          {{ const i64 crow = (i64)jc * {nd_t} + {d0 + k}; const int Lk = min(NK[crow], npad);")
                             body.append(f"            xs[{k}] = RG + crow * npad; fs[{k}] = RV + crow * npad; ds[{k}] = RM + crow * npad;")
-                            body.append(f"            Ls[{k}] = NK[crow] > npad ? 0 : Lk; }}")
-                        body.append("          double pv[2], pm[2];")
-                        body.append("          lcm_row_read_warpk<2>(xs, fs, ds, Ls, Rn, pv, pm);")
-                        body.append(f"          vals[{d0}] = pv[0]; mus[{d0}] = pm[0]; vals[{d0 + 1}] = pv[1]; mus[{d0 + 1}] = pm[1];")
+                            body.append(f"            es[{k}] = ES + crow * npad; Ls[{k}] = NK[crow] > npad ? 0 : Lk; }}")
+                        body.append(f"          lcm_row_read_win<{K}>(xs, fs, ds, es, Ls, Rn, qmin, qmax, hint + {d0}, win, vals + {d0}, mus + {d0});")
                         body.append("        }")
-                    if nd_t % 2:
-                        body.append(f"        {{ const i64 crow = (i64)jc * {nd_t} + {nd_t - 1}; const int Lk = min(NK[crow], npad);")
-                        body.append("          lcm_row_read(RG + crow * npad, RV + crow * npad, RM + crow * npad, "
-                                    f"NK[crow] > npad ? 0 : Lk, Rn, vals[{nd_t - 1}], mus[{nd_t - 1}], true); }}")
                     body.append("      } else {")
-                    body += ["  " + x.replace("{flag}", "false") for x in single]
+                    body += ["  " + x for x in single]
                     body.append("      }")
                 else:
-                    body += [x.replace("{flag}", flag) for x in single]
+                    body += single
                 if tg.taste_shocks:
                     body.append("      double vmax = -LCM_INF;")
                     body.append(f"      for (int d = 0; d < {nd_t}; ++d) vmax = vals[d] > vmax ? vals[d] : vmax;")
@@ -418,29 +435,47 @@ class EgmKernels:
         ap(f"    const int period = lcm_wi(it, {self.W_PERIOD}); const double age = lcm_wd(it, {self.W_AGE});")
         ap("    (void)period; (void)age;")
         ap(f"    const int npad = lcm_wi(it, {self.W_NPAD});")
-        ap("    const int e = (tile - tile_prefix[item]) * 256 + (int)threadIdx.x;")
-        ap(f"    if (e >= {nrow} * npad) continue;")
+        ap("    const int e_t = (tile - tile_prefix[item]) * 256 + (int)threadIdx.x;")
+        ap(f"    const bool live = e_t < {nrow} * npad;")
+        ap(f"    const int e = live ? e_t : {nrow} * npad - 1;")
         ap("    const int row = e / npad, k = e % npad;")
         body = []
         prov = dict(base_prov)
         prov.update(self._row_decode(body, "row"))
-        body.append(f"double* RC = lcm_wp<double>(it, {self.W_RC}) + (i64)row * npad;")
+        body.append(f"const double* RG = lcm_wp<const double>(it, {self.W_RG}) + (i64)row * npad;")
+        body.append(f"const double* RC = lcm_wp<const double>(it, {self.W_RC}) + (i64)row * npad;")
         body.append(f"double* RV = lcm_wp<double>(it, {self.W_RV}) + (i64)row * npad;")
         body.append(f"double* RM = lcm_wp<double>(it, {self.W_MU}) + (i64)row * npad;")
+        body.append(f"double2* ES = lcm_wp<double2>(it, {self.W_ES}) + (i64)row * npad;")
         body.append(f"const int nk = lcm_wp<const int>(it, {self.W_NK})[row];")
-        body.append("const double c = RC[k];")
-        body.append("const double cc = (c != c) ? 1.0 : c;")
         prov[id(cvar)] = "cc"
         e4 = Emitter("double", self.param_off, prov, "g")
         de = e4.emit(er.dU)
         fe = e4.emit(er.feasible)
-        body += e4.lines
-        body.append(f"double mu = (double)({de});")
-        body.append("if (c != c) mu = LCM_NAN;")
-        body.append("if (RV[k] == -LCM_INF) mu = 0.0;")
-        body.append("if (nk > npad) { RV[k] = LCM_NAN; mu = LCM_NAN; }")
-        body.append(f"if (nk == 0 || !({fe})) {{ RV[k] = -LCM_INF; mu = 0.0; }}")
-        body.append("RM[k] = mu;")
+        # value and marginal utility of node kk (the rules leave a value they
+        # have already been applied to as it is)
+        body.append("auto node = [&](int kk, double& rv, double& mu) {")
+        body.append("  const double c = RC[kk];")
+        body.append("  const double cc = (c != c) ? 1.0 : c;")
+        body += ["  " + ln for ln in e4.lines]
+        body.append("  rv = RV[kk];")
+        body.append(f"  mu = (double)({de});")
+        body.append("  if (c != c) mu = LCM_NAN;")
+        body.append("  if (rv == -LCM_INF) mu = 0.0;")
+        body.append("  if (nk > npad) { rv = LCM_NAN; mu = LCM_NAN; }")
+        body.append(f"  if (nk == 0 || !({fe})) {{ rv = -LCM_INF; mu = 0.0; }}")
+        body.append("};")
+        body.append("double rv, mu; node(k, rv, mu);")
+        body.append("double rv1 = __shfl_down_sync(0xffffffffu, rv, 1), mu1 = __shfl_down_sync(0xffffffffu, mu, 1);")
+        body.append("if (live) {")
+        body.append("  if (k + 1 < min(nk, npad)) {")
+        body.append("    if ((threadIdx.x & 31) == 31) node(k + 1, rv1, mu1);")
+        body.append("    double2 es; lcm_bracket_slopes(RG[k], RG[k + 1], rv, rv1, mu, mu1, es.x, es.y);")
+        body.append("    ES[k] = es;")
+        body.append("  }")
+        body.append("  RV[k] = rv;")
+        body.append("  RM[k] = mu;")
+        body.append("}")
         for s in body:
             ap("    " + s)
         ap("  }")

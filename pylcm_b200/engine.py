@@ -363,6 +363,8 @@ class SolvePlan:
                 "rv": torch.full((nslot, n, nrow, npad), float("nan"), **f64),
                 "mu": torch.full((nslot, n, nrow, npad), float("nan"), **f64),
                 "nk": torch.zeros((nslot, n, nrow), dtype=torch.int32, device=dev),
+                # the brackets' limited end slopes (pairs), for the continuation reads
+                "es": torch.empty((nslot, n, nrow, npad, 2), **f64),
                 "cand": [torch.empty((n, nrow, ncand), **f64) for _ in range(4)],
                 # candidate marginal utilities (the RFC envelope's tangent slopes)
                 "cm": torch.empty((n, nrow, ncand), **f64) if er.envelope == "rfc" else None,
@@ -823,6 +825,7 @@ class SolvePlan:
             r[ek.W_RC] = b["rc"][cslot, i].data_ptr()
             r[ek.W_RV] = b["rv"][cslot, i].data_ptr()
             r[ek.W_MU] = b["mu"][cslot, i].data_ptr()
+            r[ek.W_ES] = b["es"][cslot, i].data_ptr()
             r[ek.W_NK] = b["nk"][cslot, i].data_ptr()
             r[ek.W_V] = self.V[s.name][i, slot].data_ptr()
             r[ek.W_POL] = self.pol[s.name][i, slot].data_ptr()
@@ -848,12 +851,13 @@ class SolvePlan:
                         out["carry"].append((w["tm"], t.spec.name, "vmu"))
                     continue
                 if i == 0:
-                    for f in ("rg", "rv", "mu", "nk"):
+                    for f in ("rg", "rv", "mu", "nk", "es"):
                         out["carry"].append((w[f], t.spec.name, f))
                 cb = self.egm[t.spec.name]
                 r[w["rg"]] = cb["rg"][(period + 1) % 2, i].data_ptr()
                 r[w["rv"]] = cb["rv"][(period + 1) % 2, i].data_ptr()
                 r[w["mu"]] = cb["mu"][(period + 1) % 2, i].data_ptr()
+                r[w["es"]] = cb["es"][(period + 1) % 2, i].data_ptr()
                 r[w["nk"]] = cb["nk"][(period + 1) % 2, i].data_ptr()
                 r[w["npad"]] = cb["npad"]
                 r[w["taste"]] = _f2w(resolvers[i].taste_scale(t.spec.name) if t.spec.taste_shocks else 0.0)
@@ -894,7 +898,7 @@ class SolvePlan:
         G = np.repeat(tm["recs"][None], P, axis=0)
         G[:, :, ek.W_PERIOD] = pa[:, None]
         G[:, :, ek.W_AGE] = self._age_words(pa)[:, None]
-        for w, f in ((ek.W_RG, "rg"), (ek.W_RC, "rc"), (ek.W_RV, "rv"), (ek.W_MU, "mu"), (ek.W_NK, "nk")):
+        for w, f in ((ek.W_RG, "rg"), (ek.W_RC, "rc"), (ek.W_RV, "rv"), (ek.W_MU, "mu"), (ek.W_NK, "nk"), (ek.W_ES, "es")):
             G[:, :, w] = self._cptrs_many(name, f, pa)
         G[:, :, ek.W_V] = self._vptrs_many(name, pa)
         G[:, :, ek.W_POL] = self._vptrs_many(name, pa, pol=True)

@@ -107,7 +107,7 @@ def solve_bytes(eng: SolveEngine) -> int:
             solver = s.solver
             n_cand = int(solver.n_constrained_points) + len(solver.savings_grid.to_numpy())
             n_pad = int(np.ceil(solver.refined_grid_factor * n_cand))
-            b += 2 * n_rows * (4 * n_pad * 8 + 4)  # refined grid, policy, value, u'(c); counts
+            b += 2 * n_rows * (6 * n_pad * 8 + 4)  # refined grid, policy, value, u'(c), two end slopes; counts
             b += n_rows * n_cand * 8 * 4 * 2  # candidates + envelope workspace
         # expectation tables of the targets (at most one per target and target set)
         for t in specs:
