@@ -61,7 +61,9 @@ typedef struct lcmx_module lcmx_module;
  * `items` holds n_items records of 64-bit words whose layout is fixed by the
  * code generator for that kernel; `tile_prefix[i]` is the first tile of item
  * i and tile_prefix[n_items] the total tile count.  grid == 0 selects
- * (SM count x resident CTAs per SM). */
+ * (SM count x resident CTAs per SM); grid < 0, for tiles that differ in work,
+ * one CTA per tile while there are fewer than 8 per resident CTA, then the
+ * same. */
 typedef struct {
   const void* items;
   const int* tile_prefix;

@@ -360,8 +360,12 @@ static int launch_items(lcmx_module* mod, const char* kernel, const lcmx_launch_
       mod->geometry[key] = per_sm;
     }
   }
+  // uneven tiles (grid < 0): the hardware's block scheduler balances them
+  // better than the kernels' grid stride until a resident CTA has many
+  const int resident = mod->ctx->sm_count * per_sm;
   int grid = a->grid;
-  if (grid <= 0) grid = mod->ctx->sm_count * per_sm;
+  if (grid < 0) grid = a->n_tiles < 8 * resident ? a->n_tiles : resident;
+  if (grid == 0) grid = resident;
   if (grid > a->n_tiles) grid = a->n_tiles;
   const void* items = a->items;
   const int* prefix = a->tile_prefix;

@@ -128,6 +128,11 @@ class _Records:
 
 
 SM_COUNT = 148
+# grid of launches whose tiles differ in work (see lcmx_launch_args): measured
+# on the B200, grid stride / one CTA per tile: DC-EGM continuation of 12 x 777
+# points 253 / 175 us, of 32 x 2000 (18 tiles per resident CTA) 614 / 634;
+# kernel (a) in the line form, 48 x 2331 states 192 / 162 us
+UNEVEN = -1
 RESIDENT_THREADS_PER_SM = 1024
 FUES_SMEM_MAX_N = 4096  # longest candidate row of the item-form FUES launch
 ENVELOPE_MAX_N = 4096  # longest candidate row of the LTM / RFC / MSS envelope kernels
@@ -708,6 +713,8 @@ class SolvePlan:
         b.add("atab", rk, rk.atab_name(), rows, g["atab_tiles"], 256, 0, period)
         # kernel (a) reads the same records
         b.add_same_records("bellman", rk, rk.bellman_name(), g["tiles"], rk.cfg.block, rk.smem_bytes, period)
+        if rk._line is not None:
+            b.launches[-1].grid = UNEVEN
 
 
     def ensure_sim_records(self, upload: bool = True) -> None:
@@ -934,6 +941,7 @@ class SolvePlan:
         rows = g["rows"][k]
         cname, uname, pname = ek.names()
         rec.add("egm", ek, cname, rows, g["tiles_c"], 256, 0, period)
+        rec.launches[-1].grid = UNEVEN
         # FUES over every instance's candidate rows (one tile per row)
         b = self.egm[name]
         ncand = b["ncand"]

@@ -28,6 +28,7 @@ from typing import Mapping
 
 import numpy as np
 
+from pylcm_b200.engine import UNEVEN
 from pylcm_b200.exceptions import InvalidInitialConditionsError, InvalidParamsError
 from pylcm_b200.grids import DiscreteGrid
 from pylcm_b200.runtime import bundle
@@ -398,7 +399,7 @@ class SimPlan:
                     ops += self.plan.period_input_ops(period)
                     done_inputs.add(period)
                 ops.append(rk.module.prepared("sim", rk.sim_name(), ib + 8 * off, pb + 4 * poff, n_items, tiles, 256, 0,
-                                              seed=0))
+                                              grid=UNEVEN, seed=0))
             self._bundled = bundle(ops)
         for launch in self._bundled:
             launch(stream)
