@@ -22,13 +22,20 @@
 // All publish the survivors in sorted order, NaN-padded to n_out, with their
 // count (n_kept > n_out: overflow, the row holds a truncated prefix).
 //
-// GPU mapping: one CTA per row, the row staged in shared memory and sorted by
-// a bitonic sort of (monotone 64-bit grid image, input index) pairs.  The
-// CTA then walks the sorted positions in rounds of one position per thread:
-// each thread decides its position (LTM: a scan over every segment, all
-// threads reading the same segment at once -- a shared-memory broadcast; RFC:
-// 2 x search_radius neighbour tests), and a block-wide prefix sum of the
-// survivors places them in the output.  Arithmetic that the reference rounds
+// GPU mapping: one CTA per row, the row staged in shared memory and, unless it
+// is ascending already, sorted by a bitonic sort of (monotone 64-bit grid
+// image, input index) pairs.  The CTA then walks the sorted positions in
+// rounds of one position per thread: each thread decides its position (LTM: a
+// scan over the segments, all threads reading the same segment at once -- a
+// shared-memory broadcast; RFC: 2 x search_radius neighbour tests), and a
+// block-wide prefix sum of the survivors places them in the output.
+//
+// The scans are what bounds it: n^2 segment tests a row.  Candidates come
+// almost in order, so a run of 16 consecutive segments covers a short stretch
+// of the abscissae: the scans read each run's range first and test its
+// segments only where the query falls into it (any order stays correct, only
+// slower).  B200, MSS on 6 x 33 rows of 520 candidates: 258 us
+// per launch with every segment tested, 81 in runs.  Arithmetic that the reference rounds
 // step by step is written with explicitly rounded operations (no contraction
 // into fused multiply-adds), so the rows equal a step-by-step double
 // evaluation.
@@ -145,6 +152,49 @@ __device__ __forceinline__ unsigned long long env_key(double x) {
   return (b >> 63) ? ~b : (b | 0x8000000000000000ULL);
 }
 
+constexpr int kRun = 16;  // consecutive segments tested behind one range
+
+// [min, max] of the nodes of every run of kRun segments (NaN nodes aside: their
+// segments bracket nothing); the caller synchronises after
+__device__ __forceinline__ void env_run_ranges(const double* g, int n, double2* range) {
+  const double inf = __longlong_as_double(0x7ff0000000000000LL);
+  const int half = threadIdx.x & 15;
+  const int runs = (n + kRun - 2) / kRun;  // of n - 1 segments
+  for (int r = threadIdx.x >> 4; r < ((runs + 1) & ~1); r += kEnvBlock / 16) {
+    double lo = inf, hi = -inf;
+    for (int k = r * kRun + half; k <= min(r * kRun + kRun, n - 1); k += 16) {
+      lo = fmin(lo, g[k]);
+      hi = fmax(hi, g[k]);
+    }
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) {
+      lo = fmin(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+      hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+    }
+    if (half == 0 && r < runs) range[r] = make_double2(lo, hi);
+  }
+}
+
+// f(k) for the segments k of every run whose range holds q, in order, until
+// it returns true
+template <class F>
+__device__ __forceinline__ void env_each_segment(const double2* range, int n, double q, F f) {
+  for (int k0 = 0, r = 0; k0 + 1 < n; k0 += kRun, ++r) {
+    const double2 lh = range[r];
+    if (!(lh.x <= q && q <= lh.y)) continue;
+    const int k1 = min(k0 + kRun, n - 1);
+    for (int k = k0; k < k1; ++k)
+      if (f(k)) return;
+  }
+}
+
+// is (key, index) ascending already?  (for the whole CTA)
+__device__ __forceinline__ bool env_sorted(const unsigned long long* key, int n) {
+  bool ok = true;
+  for (int t = threadIdx.x; t + 1 < n; t += kEnvBlock) ok = ok && key[t] <= key[t + 1];
+  return __syncthreads_and(ok);
+}
+
 // inclusive prefix sum of one int per thread over the CTA; `tot` gets the total
 __device__ __forceinline__ int env_block_scan(int x, int* warp_sums, int& tot) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -171,19 +221,19 @@ __device__ __forceinline__ int env_block_scan(int x, int* warp_sums, int& tot) {
 __device__ __forceinline__ void env_sort(unsigned long long* key, int* idx, int np2) {
   for (int size = 2; size <= np2; size <<= 1) {
     for (int stride = size >> 1; stride > 0; stride >>= 1) {
-      for (int t = threadIdx.x; t < np2; t += kEnvBlock) {
-        const int u = t ^ stride;
-        if (u > t) {
-          const unsigned long long ka = key[t], kb = key[u];
-          const int ia = idx[t], ib = idx[u];
-          const bool a_gt = ka > kb || (ka == kb && ia > ib);
-          const bool up = (t & size) == 0;
-          if (a_gt == up) {
-            key[t] = kb;
-            key[u] = ka;
-            idx[t] = ib;
-            idx[u] = ia;
-          }
+      const int ls = __ffs(stride) - 1;  // stride = 2^ls
+      for (int j = threadIdx.x; j < (np2 >> 1); j += kEnvBlock) {
+        // the j-th pair (t, t + stride): the positions whose bit ls is clear
+        const int t = ((j >> ls) << (ls + 1)) | (j & (stride - 1)), u = t + stride;
+        const unsigned long long ka = key[t], kb = key[u];
+        const int ia = idx[t], ib = idx[u];
+        const bool a_gt = ka > kb || (ka == kb && ia > ib);
+        const bool up = (t & size) == 0;
+        if (a_gt == up) {
+          key[t] = kb;
+          key[u] = ka;
+          idx[t] = ib;
+          idx[u] = ia;
         }
       }
       __syncthreads();
@@ -195,6 +245,7 @@ template <class Rows, int KIND>
 __global__ void __launch_bounds__(kEnvBlock) envelope_kernel(Rows rows) {
   extern __shared__ __align__(16) unsigned char env_smem[];
   __shared__ int warp_sums[kEnvBlock / 32];
+  __shared__ double2 range[kEnvMaxN / kRun];
   const double nan = __longlong_as_double(0x7ff8000000000000LL);
   const double inf = __longlong_as_double(0x7ff0000000000000LL);
   const int total = rows.count();
@@ -227,8 +278,10 @@ __global__ void __launch_bounds__(kEnvBlock) envelope_kernel(Rows rows) {
       }
     }
     __syncthreads();
-    env_sort(key, idx, np2);
-    if (KIND == kRfc) {
+    if (KIND == kLtm) env_run_ranges(g, n, range);
+    const bool in_order = env_sorted(key, n);
+    if (!in_order) env_sort(key, idx, np2);
+    if (KIND == kRfc && !in_order) {
       // rows in sorted order, through the key buffer (no longer needed)
       double* tmp = reinterpret_cast<double*>(key);
       double* arrs[4] = {g, p, v, m};
@@ -252,9 +305,8 @@ __global__ void __launch_bounds__(kEnvBlock) envelope_kernel(Rows rows) {
           if (!(env_isnan(q) || env_isnan(v[i]))) {
             bool found = false;
             double bv = -inf, bp = nan;
-            double gl = g[0];
-            for (int k = 0; k + 1 < n; ++k) {
-              const double gr = g[k + 1];
+            env_each_segment(range, n, q, [&](int k) {
+              const double gl = g[k], gr = g[k + 1];
               const bool br = (gl <= gr) ? (gl <= q && q <= gr) : (gr <= q && q <= gl);
               if (br) {
                 const double vl = v[k], vr = v[k + 1];
@@ -274,8 +326,8 @@ __global__ void __launch_bounds__(kEnvBlock) envelope_kernel(Rows rows) {
                   }
                 }
               }
-              gl = gr;
-            }
+              return false;
+            });
             if (found && !(bv == -inf)) {
               keep = true;
               og = q;
@@ -304,8 +356,10 @@ __global__ void __launch_bounds__(kEnvBlock) envelope_kernel(Rows rows) {
               const double mx = (env_isnan(ag) || env_isnan(at)) ? nan : (ag > at ? ag : at);
               const double floor_ = __dmul_rn(eps16, mx);
               const bool below = gap < __dsub_rn(tan, floor_);
-              const double slope = (dg == 0.0) ? 0.0 : __ddiv_rn(__dsub_rn(p[t], p[j]), dg);
-              if (below && fabs(slope) > thr) deleted = true;
+              if (below) {
+                const double slope = (dg == 0.0) ? 0.0 : __ddiv_rn(__dsub_rn(p[t], p[j]), dg);
+                if (fabs(slope) > thr) deleted = true;
+              }
             }
             if (!deleted) {
               keep = true;
@@ -368,31 +422,34 @@ __device__ __forceinline__ bool mss_link_at(const double* g, const double* v, co
 
 // envelope value at q (-inf: no finite bracketing interpolant); `link` the
 // winner (first link within the tie band), -1 when no live link brackets q
-__device__ double mss_eval(const double* g, const double* v, const int* lseg, int n, double q, int& link) {
+__device__ double mss_eval(const double* g, const double* v, const int* lseg, const double2* range, int n, double q,
+                           int& link) {
   const double inf = __longlong_as_double(0x7ff0000000000000LL);
   double env = -inf;
   bool any = false;
-  for (int k = 0; k + 1 < n; ++k) {
+  env_each_segment(range, n, q, [&](int k) {
     double vi, rel;
     if (mss_link_at(g, v, lseg, k, q, vi, rel)) {
       any = true;
       if (isfinite(vi) && vi > env) env = vi;
     }
-  }
+    return false;
+  });
   link = -1;
   if (!any) return env;
   const double floor_ = __dmul_rn(16.0 * 2.220446049250313e-16, fmax(1.0, fabs(env)));
   const double lo = __dsub_rn(env, floor_);
-  for (int k = 0; k + 1 < n; ++k) {
+  env_each_segment(range, n, q, [&](int k) {
     double vi, rel;
     if (mss_link_at(g, v, lseg, k, q, vi, rel)) {
       const double mv = isfinite(vi) ? vi : -inf;
       if (mv >= lo) {
         link = k;
-        break;
+        return true;
       }
     }
-  }
+    return false;
+  });
   return env;
 }
 
@@ -405,6 +462,7 @@ template <class Rows>
 __global__ void __launch_bounds__(kEnvBlock) mss_kernel(Rows rows) {
   extern __shared__ __align__(16) unsigned char env_smem[];
   __shared__ int warp_sums[kEnvBlock / 32];
+  __shared__ double2 range[kEnvMaxN / kRun];
   const double nan = __longlong_as_double(0x7ff8000000000000LL);
   const double inf = __longlong_as_double(0x7ff0000000000000LL);
   const double eps16 = 16.0 * 2.220446049250313e-16;
@@ -434,7 +492,8 @@ __global__ void __launch_bounds__(kEnvBlock) mss_kernel(Rows rows) {
       key[t] = t >= n ? ~0ULL : ((env_isnan(g[t]) || env_isnan(v[t])) ? env_key(inf) : env_key(g[t]));
     }
     __syncthreads();
-    env_sort(key, idx, np2);
+    env_run_ranges(g, n, range);
+    if (!env_sorted(key, n)) env_sort(key, idx, np2);
     // links: branch ids (a running count of decreases) and liveness
     int base = 0;
     for (int k0 = 0; k0 < n - 1; k0 += kEnvBlock) {
@@ -459,7 +518,7 @@ __global__ void __launch_bounds__(kEnvBlock) mss_kernel(Rows rows) {
       const int i = idx[t];
       int link = -1;
       double e = -inf;
-      if (!(env_isnan(g[i]) || env_isnan(v[i]))) e = mss_eval(g, v, lseg, n, g[i], link);
+      if (!(env_isnan(g[i]) || env_isnan(v[i]))) e = mss_eval(g, v, lseg, range, n, g[i], link);
       const bool node = link >= 0 && !(e == -inf);
       ev[t] = e;
       wl[t] = node ? link : -1;
@@ -498,7 +557,7 @@ __global__ void __launch_bounds__(kEnvBlock) mss_kernel(Rows rows) {
             pb = __dadd_rn(p[b], __dmul_rn(psb, __dsub_rn(x, g[b])));
             if (x > qp && x < q) {
               int lk;
-              const double ce = mss_eval(g, v, lseg, n, x, lk);
+              const double ce = mss_eval(g, v, lseg, range, n, x, lk);
               cross = isfinite(ce) && isfinite(y) &&
                       fabs(__dsub_rn(ce, y)) <= __dadd_rn(1e-7, __dmul_rn(1e-5, fabs(y)));
             }
