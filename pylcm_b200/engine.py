@@ -22,6 +22,8 @@ import dataclasses
 import hashlib
 import math
 import struct
+import threading
+import weakref
 from typing import Any, Sequence
 
 import numpy as np
@@ -159,6 +161,20 @@ def default_config(spec: RegimeSpec, precision: str, n_items: int = 1) -> Launch
     return LaunchConfig(block=256, lanes=lanes, chunk=chunk, sb=sb)
 
 
+def current_stream_handle(device: int) -> int:
+    import torch
+
+    return torch.cuda.current_stream(device).cuda_stream if torch.cuda.is_available() else 0
+
+
+# Spare plans (SolveEngine.give_plan): the most device memory of one, the most
+# kept by the process, and the engines that hold one, oldest first.
+SPARE_PLAN_BYTES = 64 << 20
+SPARE_PLANS = 8
+_spare_engines: list = []
+_spare_lock = threading.Lock()
+
+
 class SolveEngine:
     """Compiles and runs the per-period kernels of one model structure."""
 
@@ -172,6 +188,7 @@ class SolveEngine:
         self._bases: dict[tuple, RegimeKernels] = {}  # before the batch's launch shape is chosen
         self._by_batch: dict[tuple, RegimeKernels] = {}  # (regime, targets, instances)
         self._traces: dict[tuple, TracedRegime] = {}
+        self._spare: SolvePlan | None = None  # the plan of a finished one-instance call
         self._targets: dict[tuple, tuple] = {}
 
     # ------------------------------------------------------------ helpers
@@ -256,6 +273,62 @@ class SolveEngine:
     def plan(self, params_list: Sequence) -> "SolvePlan":
         return SolvePlan(self, list(params_list))
 
+    # The buffers, item records and launch list of a one-instance plan are the
+    # same for every parameter set, and a call writes everything it computes
+    # anew.  Building them was 8.3 of 9.5 ms of a solve of 4 regimes over 40
+    # periods, so the plan of a finished call is kept until the next call takes
+    # it, at most SPARE_PLANS of SPARE_PLAN_BYTES each in the process.
+    def take_plan(self, params) -> "SolvePlan":
+        """A one-instance plan with `params` loaded, the caller's alone: the
+        spare one if it was built on the current stream (which then orders
+        every use of its memory), otherwise a new one."""
+        stream = current_stream_handle(self.device)
+        with _spare_lock:
+            plan = self._spare
+            if plan is not None and plan.home_stream == stream:
+                self._spare = None
+                _spare_engines[:] = [r for r in _spare_engines if r() not in (None, self)]
+            else:
+                plan = None
+        if plan is None:
+            return self.plan([params])
+        plan.set_params([params])
+        return plan
+
+    def give_plan(self, plan: "SolvePlan") -> None:
+        """Keep a plan that no queued work uses and nobody reads any more.  Not
+        with taste shocks: their scales are words of the uploaded records."""
+        if any(s.taste_shocks for s in self.specs) or plan.nbytes() > SPARE_PLAN_BYTES:
+            return
+        with _spare_lock:
+            if self._spare is not None:
+                return
+            self._spare = plan
+            _spare_engines.append(weakref.ref(self))
+            while len(_spare_engines) > SPARE_PLANS:
+                old = _spare_engines.pop(0)()
+                if old is not None:
+                    old._spare = None
+
+    def solve_host(self, params, policy: bool, collect_carries: bool = False) -> tuple[dict, dict, dict]:
+        """(V, policy, carries) of one parameter set, V and policy as host
+        arrays (policy empty unless asked for): one device->host copy per
+        regime, a period's array a view of it."""
+        plan = self.take_plan(params)
+        carries = plan.run_collecting_carries() if collect_carries else plan.run()
+        plan.check_status()
+        out: list[dict] = []
+        for buf in (plan.V, plan.pol if policy else {}):
+            res: dict = {}
+            for s in self.specs:
+                if s.name in buf:
+                    host = buf[s.name][0].cpu().numpy()  # waits for the stream
+                    for period, k in plan.slot[s.name].items():
+                        res.setdefault(period, {})[s.name] = host[k].reshape(s.state_shape)
+            out.append(dict(sorted(res.items())))
+        self.give_plan(plan)
+        return out[0], out[1], carries or {}
+
     def solve(self, params, collect_carries: bool = False):
         """(V, policy) of one parameter set; with ``collect_carries`` also
         each period's DC-EGM carry rows (see
@@ -292,6 +365,7 @@ class SolvePlan:
         self.n = n
         dev = torch.device("cuda", eng.device)
         self.dev = dev
+        self.home_stream = current_stream_handle(eng.device)
         fp32 = eng.precision == "fp32"
         resolvers = [eng.resolver(p) for p in params_list]
         self.params_list = params_list
@@ -786,6 +860,31 @@ class SolvePlan:
             if key[0] == "gs":
                 out.setdefault(g["spec"].name, []).append((g["rk"], g["rows"], g["periods"]))
         return out
+
+    def set_params(self, params_list: list) -> None:
+        """Make the plan's instances solve `params_list` (no taste shocks:
+        their scales are words of the uploaded records)."""
+        torch = self.torch
+        resolvers = [self.eng.resolver(p) for p in params_list]
+        memo: dict = {}
+        packed = {key: pack(resolvers, memo) for key, pack in self._pack_many.items() if len(key) == 2}
+        packed.update({key: self._pack_many[key](resolvers, {}) for key in self._pack_many if len(key) != 2})
+        for key, vecs in packed.items():
+            self.params[key].copy_(torch.from_numpy(np.ascontiguousarray(vecs, dtype=np.float64)))
+        self.params_list, self.resolvers = params_list, resolvers
+
+    def nbytes(self) -> int:
+        """Device bytes of the plan's buffers."""
+        total = 0
+        for d in (self.V, self.pol, self.params, self.atab, self.vmu, self.bst):
+            total += sum(t.numel() * t.element_size() for t in d.values())
+        for e64, e32, _, _ in self.ev.values():
+            total += e64.numel() * 8 + (e32.numel() * 4 if e32 is not None else 0)
+        for b in self.egm.values():
+            for t in list(b.values()) + b["cand"]:
+                if hasattr(t, "element_size"):
+                    total += t.numel() * t.element_size()
+        return total + self.items.numel() * 8 + self.prefix.numel() * 4
 
     def load_params(self, slot: int, params) -> None:
         """Make instance `slot` solve `params`: its parameter vectors (device,

@@ -108,15 +108,14 @@ class Model:
 
         validate_transitions(self, params, log_level)
         eng = self.engine(precision)
-        if return_simulation_policy:
+        if not return_device:
+            V, pol, carries = eng.solve_host(params, return_policy, collect_carries=return_simulation_policy)
+        elif return_simulation_policy:
             V, pol, carries = eng.solve(params, collect_carries=True)
         else:
             (V, pol), carries = eng.solve(params), {}
         if log_level != "off":
             _check_nan(V, raise_=(log_level == "debug"))
-        if not return_device:
-            V = {p: {r: v.cpu().numpy() for r, v in d.items()} for p, d in V.items()}
-            pol = {p: {r: v.cpu().numpy() for r, v in d.items()} for p, d in pol.items()}
         V = MappingProxyType({p: MappingProxyType(d) for p, d in V.items()})
         out = [V]
         if return_policy:

@@ -170,13 +170,13 @@ def jax_key_chain(model, params, seed: int) -> dict:
             d = {}
             if s.taste_shocks:
                 d["taste"] = key
-                key = jaxrng.split(key, 1)[0]  # the running key: counters (0, 0)
+                key = jaxrng.split_key(key, 1)[0]  # the running key: counters (0, 0)
             if not s.terminal:
-                ks = jaxrng.split(key, 3)
+                ks = jaxrng.split_key(key, 3)
                 run, d["regime"], key = ks[0], ks[1], ks[2]
                 for _, tname, state in names[s.name]:
                     d[(tname, state)] = run
-                    run = jaxrng.split(run, 1)[0]
+                    run = jaxrng.split_key(run, 1)[0]
             chain[(period, s.name)] = d
     return chain
 
@@ -435,15 +435,26 @@ def simulate(model, *, params, initial_conditions, V_arr=None, seed: int = 0, pr
     import torch
 
     eng = model.engine(precision)
-    plan = eng.plan([params])
     if V_arr is None:
+        plan = eng.take_plan(params)
         plan.run()
     else:
+        given = {(r, int(p)) for p, regs in V_arr.items() for r in regs}
+        whole = all((s.name, p) in given for s in eng.specs for p in s.active_periods)
+        # (value arrays with gaps go to a plan of their own: nothing of an earlier call is in it)
+        plan = eng.take_plan(params) if whole else eng.plan([params])
+        # one host->device copy per regime when every period is there
+        dst = {r: torch.empty(V.shape[1:], dtype=V.dtype) if whole else V[0] for r, V in plan.V.items()}
         for p, regs in V_arr.items():
             for r, v in regs.items():
                 k = plan.slot[r].get(int(p))
                 if k is not None:
-                    plan.V[r][0, k].copy_(torch.as_tensor(np.asarray(v, dtype=np.float64).reshape(-1)))
+                    dst[r][k].copy_(torch.as_tensor(np.asarray(v, dtype=np.float64).reshape(-1)))
+        if whole:
+            for r, V in plan.V.items():
+                V[0].copy_(dst[r])
     sim = SimPlan(plan, initial_conditions, seed, rng=rng, params=params)
     sim.run()
-    return sim.result(model)
+    res = sim.result(model)  # host copies; waits for the stream
+    eng.give_plan(plan)
+    return res
