@@ -3096,12 +3096,14 @@ class RegimeKernels:
 
 
     # ------------------------------------------------------------------ (b)
-    def _weight_fill(self, t: TargetPlan, block: int) -> list[str]:
-        """Lines that fill the item's weight table W[k * J + j] (double, in
-        shared memory) with a stride of `block` threads; they read the item
-        words PV (3), period (4) and age (5) through `PV`, `period`, `age`."""
+    def _weight_fill(self, t: TargetPlan, block: int, row: int | None = None) -> list[str]:
+        """Lines that fill the item's weight table W[k * row + j] (double, in
+        shared memory; rows of J unless given) with a stride of `block`
+        threads; they read the item words PV (3), period (4) and age (5)
+        through `PV`, `period`, `age`."""
         tg = t.spec
         K, J = t.K, t.J
+        row = J if row is None else row
         L = [f"for (int e = threadIdx.x; e < {K * J}; e += {block}) {{",
              f"  const int k = e / {J}; const int j = e % {J};",
              "  int kr = k;"]
@@ -3117,6 +3119,8 @@ class RegimeKernels:
         }
         for kind, kname, size in t.key_vars:
             prov[id(ir.var(kind, kname, "i"))] = f"key_{kind}_{kname}"
+        nodes = {pos: ir.var("node", tg.states[pos].name, "i") for pos in t.stoch_pos}
+        prov.update({id(v): f"jn_{tg.states[pos].name}" for pos, v in nodes.items()})
         e = Emitter("double", self.param_off, prov, "w")
         factors = []
         for pos in t.stoch_pos:
@@ -3127,8 +3131,22 @@ class RegimeKernels:
                 n = shape[0]
                 factors.append(f"PV[{off} + key_state_{law.source_process} * {n} + jn_{ax.name}]")
             else:
+                items = law.expr.items
+                first = items[0]
+                if first.op == "pidx" and all(
+                    x.op == "pidx" and x.args[0] == first.args[0] and len(x.args) == len(first.args)
+                    and all(a is b for a, b in zip(x.args[1:-1], first.args[1:-1])) and x.args[-1] is ir.const(q)
+                    for q, x in enumerate(items)
+                ):
+                    # a row of an array parameter: one read at the node's
+                    # index (a chain of selects over 32 items, one lane of a
+                    # warp per item, was most of the kernel's 100 us at
+                    # J = K = 32 and 50,000 columns)
+                    one = e.emit(ir.Expr("pidx", (*first.args[:-1], nodes[pos]), first.dtype))
+                    factors.append(f"(double)({one})")
+                    continue
                 # select item j of the Markov vector
-                exprs = [e.emit(x) for x in law.expr.items]
+                exprs = [e.emit(x) for x in items]
                 sel = exprs[-1]
                 for q in range(len(exprs) - 2, -1, -1):
                     sel = f"(jn_{ax.name} == {q} ? (double)({exprs[q]}) : {sel})"
@@ -3137,7 +3155,7 @@ class RegimeKernels:
         prod = factors[0] if factors else "1.0"
         for f_ in factors[1:]:
             prod = f"({prod}) * ({f_})"
-        L.append(f"  W[e] = {prod};")
+        L.append(f"  W[{'e' if row == J else f'k * {row} + j'}] = {prod};")
         L.append("}")
         return L
 
@@ -3165,7 +3183,7 @@ class RegimeKernels:
         NP = (K + 15) // 16 * 16
         ncol = 32 if NP <= 32 else 64 if NP <= 64 else 128 if NP <= 128 else 256
         dyn = 2 * 128 * JP * 4 + 2 * NP * JP * 4 + 128
-        static = K * J * 8 + K * 4 + 8 + 4 + 4 + 64
+        static = K * J * 8 + K * 20 + 8 + 4 + 4 + 64
         # at most 512 / ncol CTAs per SM so that every CTA's tensor-memory
         # allocation succeeds at once: pad the dynamic shared memory so that
         # no more CTAs fit (228 KB per SM, 1 KB reserved per CTA)
@@ -3202,8 +3220,24 @@ class RegimeKernels:
         tg = t.spec
         K, J = t.K, t.J
         stoch = t.stoch_pos
+        # Bounds: at a few thousand columns one chain of dependent reads (item
+        # words, values, weights); at 10^5 columns with J = K = 32 the FP64
+        # products.  So a thread reads its column's values before the weights
+        # are made (up to 16 nodes, or the first chunk of 8), two weights per
+        # shared-memory read, and 16 rows at a time (three CTAs per SM).  A
+        # value of -inf or NaN (an infeasible state; one lane of a warp is enough
+        # to send it the slow way) is taken out of the sums as a bit and put
+        # back at the end: the sum is -inf or NaN in every row that weighs it.
+        # Values of +inf, and all of them beside weights that are not finite
+        # or negative, go term by term.
         B = 256
-        KC = min(K, 32)
+        KC = min(K, 16)
+        JC = J if J <= 16 else 8
+        one = JC == J  # every value stays in registers
+        # rows of W start on 16 bytes (where the static 48 KB hold them padded)
+        JS = J + J % 2 if 8 * K * (J + 3) + 64 <= 49152 else J
+        pair = JS % 2 == 0
+        bits = K > 8 and J <= 64 and 8 * K * (JS + 2) + 64 <= 49152
         # weight expressions per stochastic axis
         L: list[str] = []
         ap = L.append
@@ -3216,11 +3250,15 @@ class RegimeKernels:
         self.e_words = 9 + len(tg.states)
         ap(f"// ---- expectation {spec.name} -> {tg.name}: K={K} J={J}")
         ap(
-            f'extern "C" __global__ void __launch_bounds__({B}) {name}('
+            f'extern "C" __global__ void __launch_bounds__({B}{', 3' if K > 16 else ''}) {name}('
             "const i64* __restrict__ items, const int* __restrict__ tile_prefix, int n_items, int n_tiles) {"
         )
-        ap(f"  __shared__ double W[{K * J}];")
+        ap(f"  __shared__ __align__(16) double W[{K * JS}];")
         ap(f"  __shared__ double Winv[{K}];")
+        if bits:
+            ap(f"  __shared__ u64 Wnz[{K}];  // nodes a row weighs")
+            ap("  __shared__ int Wodd;  // a weight is not finite or negative")
+        ap("  int cur = -1;")
         ap("  for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {")
         ap("    const int item = lcm_find_item(tile_prefix, n_items, tile);")
         ap(f"    const i64* it = items + (i64)item * {self.e_words};")
@@ -3233,51 +3271,116 @@ class RegimeKernels:
         ap("    const int cblk = lcm_wi(it, 6);")
         ap("    const int n_cols = lcm_wi(it, 7);")
         ap("    (void)period; (void)age;")
-        ap("    __syncthreads();")
-        for s_ in self._weight_fill(t, B):
-            ap("    " + s_)
-        ap("    __syncthreads();")
-        ap(f"    for (int k = threadIdx.x; k < {K}; k += {B}) {{")
-        ap(f"      double sw = 0.0; for (int j = 0; j < {J}; ++j) sw += W[k * {J} + j];")
-        ap("      Winv[k] = sw > 0.0 ? sw : 1.0;")
-        ap("    }")
-        ap("    __syncthreads();")
-        # block statistics of the float table (word BSTATS, 0: none): per row k
-        # and 16 columns, (max, finite |max|), for the search's group skipping
-        ap(f"    float2* BST = EV32 ? lcm_wp<float2>(it, {8 + len(tg.states)}) : nullptr;")
-        ap("    const int nb16 = (n_cols + 15) >> 4;")
         ap(f"    const int col_t = (tile - tile_prefix[item]) * {B} + (int)threadIdx.x;")
         ap("    const bool live = col_t < n_cols;")
         ap("    const int col = live ? col_t : 0;")
-        ap("    {")
         # decode col -> det indices + cflat ; compute base offset per j
-        ap("      const int cflat = col % cblk; int dr = col / cblk;")
-        det_names = []
+        ap("    const int cflat = col % cblk; int dr = col / cblk; (void)dr;")
         for pos in reversed(t.det_pos):
             ax = tg.states[pos]
-            ap(f"      const int di_{ax.name} = dr % {ax.size}; dr /= {ax.size};")
+            ap(f"    const int di_{ax.name} = dr % {ax.size}; dr /= {ax.size};")
         # strides over target discrete axes in order
         disc_pos = [p for p, ax in enumerate(tg.states) if ax.kind != "continuous"]
-        ap(f"      for (int k0 = 0; k0 < {K}; k0 += {KC}) {{")
-        ap(f"        double acc[{KC}];")
-        ap(f"        #pragma unroll\n        for (int kk = 0; kk < {KC}; ++kk) acc[kk] = 0.0;")
-        ap(f"        for (int j = 0; j < (live ? {J} : 0); ++j) {{")
-        ap("          int jr = j;")
+        ap("    // value of node j of this column (0 beyond the last); nodes j0 .. j0 + JC - 1")
+        ap("    auto at = [&](int j) -> double {")
+        ap("      int jr = j; (void)jr;")
         for pos in reversed(stoch):
             ax = tg.states[pos]
-            ap(f"          const int jn_{ax.name} = jr % {ax.size}; jr /= {ax.size};")
+            ap(f"      const int jn_{ax.name} = jr % {ax.size}; jr /= {ax.size};")
         off = "0"
         for pos in disc_pos:
             ax = tg.states[pos]
             iv = f"jn_{ax.name}" if pos in stoch else f"di_{ax.name}"
             off = f"({off}) * {ax.size} + {iv}"
-        ap(f"          const double v = Vt[(i64)({off}) * cblk + cflat];")
-        ap(f"          #pragma unroll\n          for (int kk = 0; kk < {KC}; ++kk) {{")
-        ap(f"            const int k = k0 + kk; if (k < {K}) acc[kk] += lcm_zs(W[k * {J} + j], v);")
+        ap(f"      return live && j < {J} ? Vt[(i64)({off}) * cblk + cflat] : 0.0;")
+        ap("    };")
+        ap(f"    auto load = [&](int j0, double (&v)[{JC}]) {{")
+        ap("      #pragma unroll")
+        ap(f"      for (int q = 0; q < {JC}; ++q) v[q] = at(j0 + q);")
+        ap("    };")
+        ap(f"    double v[{JC}]; load(0, v);")
+        ap("    if (item != cur) {  // uniform over the CTA")
+        ap("    cur = item;")
+        ap("    __syncthreads();")
+        if bits:
+            ap("    if (threadIdx.x == 0) Wodd = 0;")
+        for s_ in self._weight_fill(t, B, JS):
+            ap("    " + s_)
+        ap("    __syncthreads();")
+        ap(f"    for (int k = threadIdx.x; k < {K}; k += {B}) {{")
+        if bits:
+            ap(f"      double sw = 0.0; u64 nz = 0; bool odd = false;")
+            ap(f"      for (int j = 0; j < {J}; ++j) {{")
+            ap(f"        const double w = W[k * {JS} + j]; sw += w;")
+            ap("        if (w != 0.0) nz |= 1ull << j;")
+            ap("        odd = odd || !(w >= 0.0 && w < LCM_INF);")
+            ap("      }")
+            ap("      Wnz[k] = nz; if (odd) Wodd = 1;")
+        else:
+            ap(f"      double sw = 0.0; for (int j = 0; j < {J}; ++j) sw += W[k * {JS} + j];")
+        ap("      Winv[k] = sw > 0.0 ? sw : 1.0;")
+        ap("    }")
+        ap("    __syncthreads();")
+        ap("    }")
+        # block statistics of the float table (word BSTATS, 0: none): per row k
+        # and 16 columns, (max, finite |max|), for the search's group skipping
+        ap(f"    float2* BST = EV32 ? lcm_wp<float2>(it, {8 + len(tg.states)}) : nullptr;")
+        ap("    const int nb16 = (n_cols + 15) >> 4;")
+        ap("    {")
+        if bits:
+            ap("      u64 ninf = 0, nnan = 0;  // nodes whose value is -inf, NaN")
+        ap(f"      for (int k0 = 0; k0 < {K}; k0 += {KC}) {{")
+        ap(f"        double acc[{KC}];")
+        ap(f"        #pragma unroll\n        for (int kk = 0; kk < {KC}; ++kk) acc[kk] = 0.0;")
+        ap(f"        #pragma unroll 1\n        for (int j0 = 0; j0 < {J}; j0 += {JC}) {{")
+        if not one:
+            ap("          if (j0 > 0 || k0 > 0) load(j0, v);")
+        ap("          bool fin = true;")
+        ap(f"          #pragma unroll\n          for (int q = 0; q < {JC}; ++q) {{")
+        if bits:
+            ap("            if ((v[q] == -LCM_INF || v[q] != v[q]) && !Wodd) {")
+            ap("              (v[q] != v[q] ? nnan : ninf) |= 1ull << (j0 + q); v[q] = 0.0;")
+            ap("            }")
+        ap("            fin = fin && lcm_isfinite(v[q]);")
+        ap("          }")
+        ap("          if (fin) {")
+        ap(f"            #pragma unroll\n            for (int q = 0; q < {JC}; q += 2) {{")
+        ap(f"              #pragma unroll\n              for (int kk = 0; kk < {KC}; ++kk) {{")
+        ap(f"                const int k = k0 + kk; if (k >= {K}) continue;")
+        ap(f"                if ({int(pair)} && q + 1 < {JC} && j0 + q + 1 < {J}) {{")
+        ap(f"                  const double2 w = *reinterpret_cast<const double2*>(&W[k * {JS} + j0 + q]);")
+        ap("                  acc[kk] = __dadd_rn(acc[kk], __dmul_rn(w.x, v[q]));")
+        ap(f"                  acc[kk] = __dadd_rn(acc[kk], __dmul_rn(w.y, v[q + 1 < {JC} ? q + 1 : q]));")
+        ap("                } else {")
+        ap("                  #pragma unroll")
+        ap(f"                  for (int r = q; r < q + 2; ++r)")
+        ap(f"                    if (r < {JC} && j0 + r < {J})")
+        ap(f"                      acc[kk] = __dadd_rn(acc[kk], __dmul_rn(W[k * {JS} + j0 + r], v[r < {JC} ? r : q]));")
+        ap("                }")
+        ap("              }")
+        ap("            }")
+        ap("          } else {  // zero weights ignore a value that is not finite")
+        if one:
+            ap(f"            #pragma unroll\n            for (int j = 0; j < {J}; ++j) {{")
+            ap("              double x = v[j]; const bool nf = !lcm_isfinite(x);")
+        else:
+            ap(f"            #pragma unroll 1\n            for (int j = j0; j < min(j0 + {JC}, {J}); ++j) {{")
+            ap("              double x = at(j); const bool nf = !lcm_isfinite(x);")
+        if bits:
+            ap("              if ((ninf | nnan) >> j & 1) x = 0.0;")
+        ap(f"              #pragma unroll\n              for (int kk = 0; kk < {KC}; ++kk) {{")
+        ap(f"                const int k = k0 + kk; if (k >= {K}) continue;")
+        ap(f"                const double w = W[k * {JS} + j]; const double p = __dmul_rn(w, x);")
+        ap("                acc[kk] = __dadd_rn(acc[kk], (nf & (w == 0.0)) ? 0.0 : p);")
+        ap("              }")
+        ap("            }")
         ap("          }")
         ap("        }")
         ap(f"        #pragma unroll\n        for (int kk = 0; kk < {KC}; ++kk) {{")
         ap(f"          const int k = k0 + kk; if (k < {K}) {{")
+        if bits:
+            ap("            if (ninf & Wnz[k]) acc[kk] += -LCM_INF;")
+            ap("            if (nnan & Wnz[k]) acc[kk] = LCM_NAN;")
         ap("            const double r = acc[kk] / Winv[k];")
         ap("            if (live) {")
         ap("              EV64[(i64)k * n_cols + col] = r;")

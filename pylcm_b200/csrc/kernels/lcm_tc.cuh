@@ -173,6 +173,11 @@ __device__ __forceinline__ void lcm_tc_expect(const i64* __restrict__ items, con
   extern __shared__ unsigned char lcm_dsmem[];
   __shared__ double Wd[K * J];
   __shared__ float Wscale[K];
+  __shared__ double Wsum[K];
+  // nodes row k weighs, where the static 48 KB hold them
+  constexpr bool BITS = K > 8 && K * (8 * J + 20) + 256 <= 49152;
+  __shared__ u64 Wnz[BITS ? K : 1];
+  __shared__ int Wodd;  // a weight is negative or not finite
   __shared__ __align__(8) u64 mbar;
   __shared__ u32 tmem_slot;
   __shared__ int cur_item;
@@ -202,15 +207,41 @@ __device__ __forceinline__ void lcm_tc_expect(const i64* __restrict__ items, con
   for (int tile = blockIdx.x; tile < n_tiles && !failed; tile += gridDim.x) {
     const int item = lcm_find_item(tile_prefix, n_items, tile);
     const i64* it = items + (i64)item * e_words;
+    const double* __restrict__ Vt = lcm_wp<const double>(it, 0);
+    float* __restrict__ EV32 = lcm_wp<float>(it, 2);
+    const i64 cblk = lcm_wi(it, 6);
+    const int n_cols = lcm_wi(it, 7);
+    const int col = (tile - tile_prefix[item]) * LCM_TC_M + tid;
+    const bool live = col < n_cols;
+    // this thread's column, read ahead of the weights (up to 32 nodes)
+    constexpr int JV = J <= 32 ? J : 1;
+    double vcol[JV];
+    if constexpr (J <= 32) {
+#pragma unroll
+      for (int j = 0; j < J; ++j) vcol[j] = live ? Vt[(i64)j * cblk + col] : 0.0;
+    }
     // ---- weights of this item: FP64 table, row scales, B = W^T split in two
     if (item != cur_item) {
       __syncthreads();  // every thread is past the previous tile's reads of B / W
+      if (tid == 0) Wodd = 0;
       wfill(it, Wd);
       __syncthreads();
       for (int k = tid; k < K; k += LCM_TC_THREADS) {
         double sw = 0.0;
-        for (int j = 0; j < J; ++j) sw += Wd[k * J + j];
-        Wscale[k] = (float)(1.0 / (sw > 0.0 ? sw : 1.0));
+        u64 nz = 0;
+        bool odd = false;
+        for (int j = 0; j < J; ++j) {
+          const double w = Wd[k * J + j];
+          sw += w;
+          if constexpr (BITS) {
+            if (w != 0.0) nz |= 1ull << j;
+            odd = odd || !(w >= 0.0 && lcm_isfinite(w));
+          }
+        }
+        if constexpr (BITS) Wnz[k] = nz;
+        Wsum[k] = sw > 0.0 ? sw : 1.0;
+        Wscale[k] = (float)(1.0 / Wsum[k]);
+        if (odd) Wodd = 1;  // (BITS only)
       }
       for (int e = tid; e < NP * JP; e += LCM_TC_THREADS) {
         const int n = e / JP, j = e % JP;
@@ -222,14 +253,10 @@ __device__ __forceinline__ void lcm_tc_expect(const i64* __restrict__ items, con
       }
       if (tid == 0) cur_item = item;
     }
-    const double* __restrict__ Vt = lcm_wp<const double>(it, 0);
-    float* __restrict__ EV32 = lcm_wp<float>(it, 2);
-    const i64 cblk = lcm_wi(it, 6);
-    const int n_cols = lcm_wi(it, 7);
-    const int col = (tile - tile_prefix[item]) * LCM_TC_M + tid;
-    const bool live = col < n_cols;
     // ---- A: this thread's column, split, four reduction values per store
     bool nonfinite = false;
+    u64 ninf = 0, nnan = 0;  // nodes of value -inf and NaN, while every other one is finite
+    bool other = false;
 #pragma unroll
     for (int c = 0; c < KC; ++c) {
       u32 h[4], l[4];
@@ -237,9 +264,16 @@ __device__ __forceinline__ void lcm_tc_expect(const i64* __restrict__ items, con
       for (int q = 0; q < 4; ++q) {
         const int j = c * 4 + q;
         double v = 0.0;
-        if (live && j < J) v = Vt[(i64)j * cblk + col];
+        if constexpr (J <= 32) {
+          if (j < J) v = vcol[j < JV ? j : 0];
+        } else if (live && j < J) {
+          v = Vt[(i64)j * cblk + col];
+        }
         if (!lcm_isfinite(v)) {
           nonfinite = true;
+          if (BITS && v == -LCM_INF) ninf |= 1ull << j;
+          else if (BITS && v != v) nnan |= 1ull << j;
+          else other = true;
           v = 0.0;
         }
         lcm_tf32_split(v, h[q], l[q]);
@@ -247,6 +281,9 @@ __device__ __forceinline__ void lcm_tc_expect(const i64* __restrict__ items, con
       const u32 off = lcm_kmajor_off(tid, c * 4, LCM_TC_M);
       *reinterpret_cast<uint4*>(a_hi + off) = make_uint4(h[0], h[1], h[2], h[3]);
       *reinterpret_cast<uint4*>(a_lo + off) = make_uint4(l[0], l[1], l[2], l[3]);
+    }
+    if constexpr (BITS) {
+      if (other || Wodd) ninf = nnan = 0;
     }
     lcm_fence_async_smem();  // generic-proxy writes -> visible to the tensor core
     __syncthreads();
@@ -292,19 +329,45 @@ __device__ __forceinline__ void lcm_tc_expect(const i64* __restrict__ items, con
         float d[16];
         lcm_tmem_ld16(lane_base + (u32)n0, d);
 #pragma unroll
+        for (int q = 0; q < 16; ++q)
+          if (n0 + q < K) d[q] *= Wscale[n0 + q];
+        if (live && nonfinite) {  // FP64, zero-safe, one read of a node for 16 rows
+          double num[16];
+#pragma unroll
+          for (int q = 0; q < 16; ++q) num[q] = 0.0;
+          if (BITS && (ninf | nnan)) {  // the sum of the others, -inf or NaN in the rows that weigh such a node
+#pragma unroll 1
+            for (int j = 0; j < J; ++j) {
+              const double x = ((ninf | nnan) >> j & 1) ? 0.0 : Vt[(i64)j * cblk + col];
+#pragma unroll
+              for (int q = 0; q < 16; ++q)
+                if (n0 + q < K) num[q] = __dadd_rn(num[q], __dmul_rn(Wd[(n0 + q) * J + j], x));
+            }
+#pragma unroll
+            for (int q = 0; q < 16; ++q) {
+              if (n0 + q >= K) continue;
+              const u64 nz = Wnz[BITS ? n0 + q : 0];
+              if (ninf & nz) num[q] += -LCM_INF;
+              if (nnan & nz) num[q] = LCM_NAN;
+            }
+          } else {
+#pragma unroll 1
+            for (int j = 0; j < J; ++j) {
+              const double x = Vt[(i64)j * cblk + col];
+#pragma unroll
+              for (int q = 0; q < 16; ++q)
+                if (n0 + q < K) num[q] = __dadd_rn(num[q], lcm_zs(Wd[(n0 + q) * J + j], x));
+            }
+          }
+#pragma unroll
+          for (int q = 0; q < 16; ++q)
+            if (n0 + q < K) d[q] = (float)(num[q] / Wsum[n0 + q]);
+        }
+#pragma unroll
         for (int q = 0; q < 16; ++q) {
           const int k = n0 + q;
           if (k >= K) continue;
-          float e = d[q] * Wscale[k];
-          if (live && nonfinite) {  // FP64, zero-safe, node by node
-            double num = 0.0, sw = 0.0;
-            for (int j = 0; j < J; ++j) {
-              const double w = Wd[k * J + j];
-              sw += w;
-              num += lcm_zs(w, Vt[(i64)j * cblk + col]);
-            }
-            e = (float)(num / (sw > 0.0 ? sw : 1.0));
-          }
+          const float e = d[q];
           if (live) EV32[(i64)k * n_cols + col] = e;
           if (BST) {  // uniform over the CTA (one item per tile)
             const float2 st = lcm_block16_stats(live ? e : -lcm_lim<float>::inf());
