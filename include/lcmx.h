@@ -93,6 +93,11 @@ const char* lcmx_last_error(const lcmx_ctx* ctx);
 /* Device facts used for grid sizing and HBM admission. */
 int lcmx_device_info(lcmx_ctx* ctx, int* sm_count, size_t* free_bytes, size_t* total_bytes);
 
+/* A stream of its own that does not wait for the default stream (branches of a
+ * capture), and its end. */
+int lcmx_stream_create(lcmx_ctx* ctx, void** out);
+int lcmx_stream_destroy(lcmx_ctx* ctx, void* stream);
+
 /* Compile CUDA C for sm_100a with NVRTC and load it.  `key` names the source
  * in the in-process and on-disk cubin caches; `options` is a '\n'-separated
  * list of extra NVRTC options (may be NULL). */

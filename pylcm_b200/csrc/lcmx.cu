@@ -153,6 +153,23 @@ extern "C" int lcmx_device_info(lcmx_ctx* ctx, int* sm_count, size_t* free_bytes
   return LCMX_OK;
 }
 
+extern "C" int lcmx_stream_create(lcmx_ctx* ctx, void** out) {
+  if (!ctx || !out) return set_err(ctx, LCMX_ERR_ARGS, "lcmx_stream_create: NULL argument");
+  cudaSetDevice(ctx->device);
+  cudaStream_t s = nullptr;
+  cudaError_t e = cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking);
+  if (e != cudaSuccess) return set_err(ctx, LCMX_ERR_CUDA, std::string("cudaStreamCreateWithFlags: ") + cudaGetErrorString(e));
+  *out = s;
+  return LCMX_OK;
+}
+
+extern "C" int lcmx_stream_destroy(lcmx_ctx* ctx, void* stream) {
+  if (!ctx || !stream) return set_err(ctx, LCMX_ERR_ARGS, "lcmx_stream_destroy: NULL argument");
+  cudaError_t e = cudaStreamDestroy((cudaStream_t)stream);
+  if (e != cudaSuccess) return set_err(ctx, LCMX_ERR_CUDA, std::string("cudaStreamDestroy: ") + cudaGetErrorString(e));
+  return LCMX_OK;
+}
+
 // ---------------------------------------------------------------- caching
 static std::string cache_dir() {
   const char* d = getenv("LCMX_CACHE_DIR");

@@ -52,6 +52,7 @@ class Launch:
     smem: int
     period: int
     grid: int = 0  # CTAs of the launch (0: SM count x resident CTAs per SM)
+    regime: str = ""  # whose step of the period the launch belongs to
 
 
 class _Records:
@@ -526,12 +527,15 @@ class SolvePlan:
         b = _Records()
         ages = model.ages.values
         for period, s, targets, rk in step_list:
+            first = len(b.launches)
             if not isinstance(rk, RegimeKernels):
                 self._egm_launches(rk, period, s, targets, float(ages[period]), resolvers, b)
-                continue
-            self._gs_launches(b, rk, period, s, targets, (s.name, targets))
-            if (s.name, period) in self._vmu_need:
-                self._vmu_launch(b, s, targets, period)
+            else:
+                self._gs_launches(b, rk, period, s, targets, (s.name, targets))
+                if (s.name, period) in self._vmu_need:
+                    self._vmu_launch(b, s, targets, period)
+            for l in b.launches[first:]:
+                l.regime = s.name
         self.launches = b.launches
         self._rec = b
         for rk in {id(l.module): l.module for l in self.launches if l.kind not in ("fues", "env")}.values():
@@ -1223,9 +1227,80 @@ class SolvePlan:
         with torch.cuda.stream(s):
             self.run(s.cuda_stream)  # warm-up (module attributes, caches)
         torch.cuda.current_stream(self.dev).wait_stream(s)
-        with torch.cuda.graph(g):
-            self.run(torch.cuda.current_stream(self.dev).cuda_stream)
+        from pylcm_b200.runtime import get_context, side_streams
+
+        lanes = self._lanes()
+        with side_streams(get_context(self.eng.device), max(lanes)) as side:
+            with torch.cuda.graph(g):
+                self._run_branches(lanes, [torch.cuda.current_stream(self.dev), *side])
         self.graph = g
+
+    # The launches of one period that do not depend on one another become
+    # parallel branches of the graph: the regimes' steps (they read the next
+    # period's values and write their own regime's buffers) and, within a
+    # grid-search step, its expectations and action table before kernel (a).
+    # Most of these launches leave the GPU mostly idle (7 to 14 us each at
+    # 1.5 us of work).  The tensor-core expectations stay in one branch: a CTA
+    # holds tensor memory, and another launch's CTAs would wait for it.
+    MAX_LANES = 8
+
+    def _lanes(self) -> list[int]:
+        """The branch (0: the capturing stream) of every launch: the step's
+        own, or another one for what its kernel (a) waits for."""
+        order = {s.name: k for k, s in enumerate(self.eng.specs)}
+        tc = 1 + len(order)
+        out: list[int] = []
+        free = 0
+        for k, l in enumerate(self.launches):
+            if k == 0 or l.period != self.launches[k - 1].period:
+                free = tc + 1
+            if l.kind == "expect_tc":
+                lane = tc
+            elif l.kind == "expect":
+                lane, free = free, free + 1
+            elif l.kind == "stats":
+                lane = out[-1]  # reads what the launch before it wrote
+            else:
+                lane = 1 + order[l.regime]
+            out.append(lane)
+        # numbered without gaps, the first on the capturing stream
+        names = {lane: min(k, self.MAX_LANES - 1) for k, lane in enumerate(dict.fromkeys(out))}
+        return [names[lane] for lane in out]
+
+    def _run_branches(self, lanes: list, streams: list) -> None:
+        """Issue every launch on the stream of its lane, with the waits that
+        keep the order within a step and between periods."""
+        prepared = self._prepared
+        k, n = 0, len(prepared)
+        while k < n:  # one period
+            end = k
+            while end < n and self.launches[end].period == self.launches[k].period:
+                end += 1
+            used = list(dict.fromkeys(lanes[k:end]))
+            start = streams[0].record_event()
+            for lane in used:
+                if lane:
+                    streams[lane].wait_event(start)
+            while k < end:  # one step
+                stop = k
+                while stop < end and self.launches[stop].regime == self.launches[k].regime:
+                    stop += 1
+                before: list = []  # lanes the step's own launches wait for
+                for q in range(k, stop):
+                    lane = lanes[q]
+                    if self.launches[q].kind in ("expect", "expect_tc", "stats"):
+                        if lane not in before:
+                            before.append(lane)
+                    elif self.launches[q].kind != "atab":
+                        for b in before:
+                            if b != lane:
+                                streams[lane].wait_event(streams[b].record_event())
+                        before = []
+                    prepared[q](streams[lane].cuda_stream)
+                k = stop
+            for lane in used:
+                if lane:
+                    streams[0].wait_event(streams[lane].record_event())
 
     def run_graph(self) -> None:
         if self.graph is None:

@@ -6,6 +6,7 @@ fallback: if the library or a GPU is missing, solving raises.
 
 from __future__ import annotations
 
+import contextlib
 import ctypes
 import threading
 from collections.abc import Callable
@@ -39,6 +40,8 @@ EXPORTED = (
     "lcmx_mss_scan",
     "lcmx_envelope_step",
     "lcmx_launch_list",
+    "lcmx_stream_create",
+    "lcmx_stream_destroy",
 )
 
 
@@ -90,6 +93,8 @@ def load_library() -> ctypes.CDLL:
             "lcmx_ctx_destroy": ([vp], ip),
             "lcmx_last_error": ([vp], cp),
             "lcmx_device_info": ([vp, ctypes.POINTER(ip), ctypes.POINTER(ctypes.c_size_t), ctypes.POINTER(ctypes.c_size_t)], ip),
+            "lcmx_stream_create": ([vp, ctypes.POINTER(vp)], ip),
+            "lcmx_stream_destroy": ([vp, vp], ip),
             "lcmx_module_compile": ([vp, cp, cp, cp, ctypes.POINTER(vp)], ip),
             "lcmx_module_destroy": ([vp], ip),
             "lcmx_occupancy": ([vp, cp, ip, ip, ctypes.POINTER(ip)], ip),
@@ -254,6 +259,24 @@ class Module:
     def egm_step(self, kernel, items_ptr, prefix_ptr, n_items, n_tiles, block, smem, stream, grid=0) -> None:
         a = self._args(items_ptr, prefix_ptr, n_items, n_tiles, block, smem, grid)
         self.ctx.check(self.ctx.lib.lcmx_egm_step(self.h, kernel.encode(), ctypes.byref(a), stream))
+
+
+@contextlib.contextmanager
+def side_streams(ctx: Context, n: int):
+    """`n` streams of nobody else's (torch's come from a shared pool), as torch
+    streams, for the branches of a capture."""
+    import torch
+
+    handles = []
+    try:
+        for _ in range(n):
+            h = ctypes.c_void_p()
+            ctx.check(ctx.lib.lcmx_stream_create(ctx.h, ctypes.byref(h)))
+            handles.append(h)
+        yield [torch.cuda.ExternalStream(h.value, device=torch.device("cuda", ctx.device)) for h in handles]
+    finally:
+        for h in handles:
+            ctx.lib.lcmx_stream_destroy(ctx.h, h)
 
 
 _contexts: dict[int, Context] = {}
