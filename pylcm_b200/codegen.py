@@ -3229,7 +3229,10 @@ class RegimeKernels:
         # to send it the slow way) is taken out of the sums as a bit and put
         # back at the end: the sum is -inf or NaN in every row that weighs it.
         # Values of +inf, and all of them beside weights that are not finite
-        # or negative, go term by term.
+        # or negative, go term by term.  B200, a launch: 7 nodes x 500 columns
+        # 6.9 -> 5.0 us, of 256 instances 10.8 -> 9.0; 32 nodes x 100,000
+        # columns 99 -> 86, 16 x 81,000 30 -> 22 (with the reads but without
+        # the bits).
         B = 256
         KC = min(K, 16)
         JC = J if J <= 16 else 8
