@@ -976,9 +976,6 @@ class RegimeKernels:
 
     # (state, action) pairs of a batch from which the line form pays
     LINE_MIN_PAIRS = 16_000_000
-    # ... with collapsed rows (two axes): pairs, scanned actions, states of a
-    # line, lines
-    LINE_MIN_PAIRS_2, LINE_MIN_SCAN_2, LINE_MIN_STATES_2, LINE_MIN_LINES_2 = 120_000_000, 144, 256, 592
 
     def line_config(self, n_items: int) -> LaunchConfig:
         """The launch shape of kernel (a) for `n_items` instances where the
@@ -991,44 +988,36 @@ class RegimeKernels:
         single-precision search over one continuous action and one axis keeps
         the line form at every size (3500 x 1000: 0.71 / 0.68).
 
-        Two axes: the full search reads few rows and is hard to beat; the line
-        form needs many scanned actions to skip, lines that fill a CTA and at
-        least two waves of them, whose costs differ by a factor of three
-        (microseconds per launch, full / line, single and double precision;
-        wealth x human capital x shock x consumption of 2 or 3 instances:
-        1000 x 50 x 16 x 300 2400 / 1195 and 3608 / 1704; 413 x 23 x 11 x 157
-        470 / 283 and 651 / 409; 300 x 40 x 16 x 200 869 / 592 and 946 / 917;
-        but 587 x 28 x 32 x 136 1250 / 1233 and 1721 / 1861; 900 x 30 x 8 x 73
-        353 / 343 and 410 / 507; 136 x 26 x 7 x 226 128 / 206 and 194 / 314;
-        1000 x 13 x 4 x 300, 104 lines, 225 / 374 and 343 / 687).
+        Two axes (collapsed rows): the full search.  The line form is up to
+        twice as fast on large batches while the values are finite (1000 x 50 x
+        16 x 300, 2 instances, 2400 / 1195 us per launch), but a NaN bound
+        never skips: over 60 periods, where NaN values spread over the human
+        capital model's grid, it takes 98.7 against 63.3 ms per launch (32
+        instances of 1000 x 50 x 32 x 300, single precision) and 8.0 against
+        4.0 (one, double).  On short lines, few lines or few scanned actions
+        it loses at once (136 x 26 x 7 x 226, 128 / 206).  A launch shape that
+        is asked for (`configs`) takes it as before.
 
         Threads per state: one, or more while the states do not fill the GPU
         (21,000 states: 1 / 2 / 4 threads 1.34 / 0.95 / 0.90 ms; 70,000:
         1.55 / 1.63 / 1.77).  Strips per CTA: a CTA that walks the whole line
         builds its rows once, more CTAs fill the last wave better; the cheaper
         of the two by waves x (strips + build), the build worth a third of a
-        strip, or two thirds with collapsed rows (280 lines of 500: 2 strips
-        2.18, 1 strip 2.70 ms; 140 lines: 1.82, 1.55)."""
+        strip (280 lines of 500: 2 strips 2.18, 1 strip 2.70 ms; 140 lines:
+        1.82, 1.55)."""
         cfg, spec = self.cfg, self.spec
         if self._line is None:
             return cfg
         total = spec.n_states * n_items
-        pairs = total * spec.n_actions
+        one = len(self._line["cacts"]) == 1
+        two = any(x["coll"] for x in self._line["targets"].values())
+        if two or (total * spec.n_actions < self.LINE_MIN_PAIRS and not (one and self.precision == "fp32")):
+            return dataclasses.replace(cfg, prune=False)
         nline = spec.states[self._line["kline"]].size
         lines = spec.n_states // nline * n_items
-        two = any(x["coll"] for x in self._line["targets"].values())
-        if two:
-            pays = (pairs >= self.LINE_MIN_PAIRS_2 and nline >= self.LINE_MIN_STATES_2
-                    and lines >= self.LINE_MIN_LINES_2
-                    and spec.actions[self._line["kscan"]].size >= self.LINE_MIN_SCAN_2)
-        else:
-            one = len(self._line["cacts"]) == 1
-            pays = pairs >= self.LINE_MIN_PAIRS or (one and self.precision == "fp32")
-        if not pays:
-            return dataclasses.replace(cfg, prune=False)
         lanes = next((k for k, n in ((1, 60_000), (2, 30_000), (4, 12_000), (8, 6_000)) if total >= n), 16)
         most = math.ceil(nline / (cfg.block // lanes))
-        build = 0.67 if two else 0.35
+        build = 0.35
 
         def cost(k: int) -> float:
             return math.ceil(lines * math.ceil(most / k) / (2 * 148)) * (k + build)

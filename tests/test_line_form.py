@@ -109,15 +109,8 @@ def test_line_form_equals_the_full_search(case, lanes, sb, precision):
 
 
 @pytest.mark.parametrize("precision", ["fp32", "fp64"])
-@pytest.mark.parametrize("n_items,shape,line", [
-    (2, (1000, 50, 32, 300), True),
-    (3, (413, 23, 11, 157), True),
-    (3, (255, 40, 32, 300), False),   # lines shorter than a CTA
-    (3, (587, 28, 32, 136), False),   # few actions to skip
-    (1, (1000, 16, 32, 300), False),  # few lines
-    (2, (413, 23, 11, 157), False),   # few pairs
-])
-def test_two_axes_take_the_line_form_where_it_pays(precision, n_items, shape, line):
+@pytest.mark.parametrize("shape", [(1000, 50, 32, 300), (136, 26, 7, 226)])
+def test_two_axes_take_the_full_search_unless_asked(precision, shape):
     nw, nh, ns, nc = shape
-    rk = _rk(M.hc_model(3, nw, nh, ns, nc), M.hc_params(0, ns), precision, "alive", n_items)
-    assert (rk._line is not None) == line
+    assert _rk(M.hc_model(3, nw, nh, ns, nc), M.hc_params(0, ns), precision, "alive", 3)._line is None
+    assert _rk(M.hc_model(3, nw, nh, ns, nc), M.hc_params(0, ns), precision, "alive", 3, lanes=2)._line is not None
