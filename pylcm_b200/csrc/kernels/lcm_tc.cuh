@@ -339,8 +339,12 @@ __device__ __forceinline__ void lcm_tc_expect(const i64* __restrict__ items, con
 #pragma unroll
           for (int q = 0; q < 16; ++q) num[q] = 0.0;
           if (BITS && (ninf | nnan)) {  // the sum of the others, -inf or NaN in the rows that weigh such a node
-#pragma unroll 1
-            for (int j = 0; j < J; ++j) {
+            bool every = true;  // no row needs the sum
+#pragma unroll
+            for (int q = 0; q < 16; ++q)
+              if (n0 + q < K) every = every && ((ninf | nnan) & Wnz[BITS ? n0 + q : 0]);
+#pragma unroll 4
+            for (int j = 0; j < (every ? 0 : J); ++j) {
               const double x = ((ninf | nnan) >> j & 1) ? 0.0 : Vt[(i64)j * cblk + col];
 #pragma unroll
               for (int q = 0; q < 16; ++q)
