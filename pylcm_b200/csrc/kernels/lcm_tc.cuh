@@ -285,11 +285,11 @@ __device__ __forceinline__ void lcm_tc_expect(const i64* __restrict__ items, con
       *reinterpret_cast<uint4*>(a_hi + off) = make_uint4(h[0], h[1], h[2], h[3]);
       *reinterpret_cast<uint4*>(a_lo + off) = make_uint4(l[0], l[1], l[2], l[3]);
     }
-    if constexpr (BITS) {
-      if (other || Wodd) ninf = nnan = 0;
-    }
     lcm_fence_async_smem();  // generic-proxy writes -> visible to the tensor core
     __syncthreads();
+    if constexpr (BITS) {
+      if (other || Wodd) ninf = nnan = 0;  // (behind the barrier: a few threads of the item's first tile set Wodd)
+    }
     // ---- D = Ahi Bhi + Ahi Blo + Alo Bhi, issued by one thread
     if (tid == 0) {
       lcm_tc_fence_after();
