@@ -127,9 +127,12 @@ __device__ __forceinline__ void lcm_tmem_free(u32 taddr, u32 ncols) {
   asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
 }
 
-// 16 consecutive 32-bit TMEM columns of this thread's lane
+// 16 consecutive 32-bit TMEM columns of this thread's lane.  The load is a
+// collective of the converged warp; the epilogue's lanes part between two of
+// them (a lane whose column is not finite sums it again), so they meet here.
 __device__ __forceinline__ void lcm_tmem_ld16(u32 taddr, float* v) {
   u32 r[16];
+  __syncwarp();
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
       "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
