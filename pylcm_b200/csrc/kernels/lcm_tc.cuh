@@ -179,12 +179,14 @@ __device__ __forceinline__ void lcm_tc_expect(const i64* __restrict__ items, con
   extern __shared__ unsigned char lcm_dsmem[];
   __shared__ double Wd[K * J];
   __shared__ float Wscale[K];
-  __shared__ double Wsum[K];
-  // nodes row k weighs, where the static 48 KB hold them
+  // weight sums, and the nodes a row weighs, where the static 48 KB hold them
+  // beside the weights (a table that fills them is summed again per use)
+  constexpr bool SUMS = K * (8 * J + 12) + 256 <= 49152;
   constexpr bool BITS = K > 8 && K * (8 * J + 20) + 256 <= 49152;
-  __shared__ u64 Wnz[BITS ? K : 1];
-  __shared__ int Wodd;  // a weight is negative or not finite
-  __shared__ __align__(8) u64 mbar;
+  __shared__ __align__(8) u64 words[(SUMS ? K : 0) + (BITS ? K + 1 : 0) + 1];
+  double* const Wsum = reinterpret_cast<double*>(words);
+  u64* const Wnz = words + (SUMS ? K : 0);
+  u64& Wodd = words[BITS ? (SUMS ? 2 * K : K) : 0];  // (BITS) a weight is negative or not finite
   __shared__ u32 tmem_slot;
   __shared__ int cur_item;
 
@@ -195,7 +197,17 @@ __device__ __forceinline__ void lcm_tc_expect(const i64* __restrict__ items, con
   unsigned char* b_lo = b_hi + S::B_BYTES;
   const int tid = threadIdx.x;
   const int warp = tid >> 5;
-  const u32 bar = lcm_smem_u32(&mbar);
+  const u32 bar = lcm_smem_u32(words + sizeof(words) / 8 - 1);  // the mbarrier
+  auto wsum = [&](int k) {
+    if constexpr (SUMS) {
+      return Wsum[k];
+    } else {
+      double sw = 0.0;
+#pragma unroll 1
+      for (int j = 0; j < J; ++j) sw += Wd[k * J + j];
+      return sw > 0.0 ? sw : 1.0;
+    }
+  };
 
   if (warp == 0) lcm_tmem_alloc(lcm_smem_u32(&tmem_slot), (u32)S::NCOL);
   if (tid == 0) {
@@ -229,7 +241,9 @@ __device__ __forceinline__ void lcm_tc_expect(const i64* __restrict__ items, con
     // ---- weights of this item: FP64 table, row scales, B = W^T split in two
     if (item != cur_item) {
       __syncthreads();  // every thread is past the previous tile's reads of B / W
-      if (tid == 0) Wodd = 0;
+      if constexpr (BITS) {
+        if (tid == 0) Wodd = 0;
+      }
       wfill(it, Wd);
       __syncthreads();
       for (int k = tid; k < K; k += LCM_TC_THREADS) {
@@ -244,10 +258,13 @@ __device__ __forceinline__ void lcm_tc_expect(const i64* __restrict__ items, con
             odd = odd || !(w >= 0.0 && lcm_isfinite(w));
           }
         }
-        if constexpr (BITS) Wnz[k] = nz;
-        Wsum[k] = sw > 0.0 ? sw : 1.0;
-        Wscale[k] = (float)(1.0 / Wsum[k]);
-        if (odd) Wodd = 1;  // (BITS only)
+        sw = sw > 0.0 ? sw : 1.0;
+        if constexpr (SUMS) Wsum[k] = sw;
+        Wscale[k] = (float)(1.0 / sw);
+        if constexpr (BITS) {
+          Wnz[k] = nz;
+          if (odd) Wodd = 1;
+        }
       }
       for (int e = tid; e < NP * JP; e += LCM_TC_THREADS) {
         const int n = e / JP, j = e % JP;
@@ -291,7 +308,7 @@ __device__ __forceinline__ void lcm_tc_expect(const i64* __restrict__ items, con
     lcm_fence_async_smem();  // generic-proxy writes -> visible to the tensor core
     __syncthreads();
     if constexpr (BITS) {
-      if (other || Wodd) ninf = nnan = 0;  // (behind the barrier: a few threads of the item's first tile set Wodd)
+      if (other || Wodd) ninf = nnan = 0;  // (behind the barrier: a few threads of the item's first tile set it)
     }
     // ---- D = Ahi Bhi + Ahi Blo + Alo Bhi, issued by one thread
     if (tid == 0) {
@@ -371,7 +388,7 @@ __device__ __forceinline__ void lcm_tc_expect(const i64* __restrict__ items, con
           }
 #pragma unroll
           for (int q = 0; q < 16; ++q)
-            if (n0 + q < K) d[q] = (float)(num[q] / Wsum[n0 + q]);
+            if (n0 + q < K) d[q] = (float)(num[q] / wsum(n0 + q));
         }
 #pragma unroll
         for (int q = 0; q < 16; ++q) {
