@@ -571,6 +571,16 @@ __device__ __forceinline__ int lcm_row_bracket(const double* __restrict__ xp, in
   return lo - 1;
 }
 
+// Accesses to a value that another thread of the launch may read or store.
+__device__ __forceinline__ double lcm_ld_relaxed(const double* p) {
+  double v;
+  asm volatile("ld.relaxed.gpu.global.f64 %0, [%1];" : "=d"(v) : "l"(__cvta_generic_to_global(p)) : "memory");
+  return v;
+}
+__device__ __forceinline__ void lcm_st_relaxed(double* p, double v) {
+  asm volatile("st.relaxed.gpu.global.f64 [%0], %1;" ::"l"(__cvta_generic_to_global(p)), "d"(v) : "memory");
+}
+
 // The limited end slopes (Fritsch & Carlson) of the cubic on a bracket, as
 // lcm_bracket_read uses them: they depend on the bracket alone, so a carry row
 // keeps them beside its nodes.  LCM_LINEAR in e0 marks a bracket read linearly

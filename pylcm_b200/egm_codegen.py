@@ -452,13 +452,15 @@ class EgmKernels:
         e4 = Emitter("double", self.param_off, prov, "g")
         de = e4.emit(er.dU)
         fe = e4.emit(er.feasible)
-        # value and marginal utility of node kk (the rules leave a value they
-        # have already been applied to as it is)
+        # value and marginal utility of node kk.  A warp's last lane reads the
+        # next warp's first value, which that warp may have completed and
+        # stored already: the rules leave a value they have been applied to as
+        # it is, and the accesses are relaxed atomics of the device
         body.append("auto node = [&](int kk, double& rv, double& mu) {")
         body.append("  const double c = RC[kk];")
         body.append("  const double cc = (c != c) ? 1.0 : c;")
         body += ["  " + ln for ln in e4.lines]
-        body.append("  rv = RV[kk];")
+        body.append("  rv = lcm_ld_relaxed(RV + kk);")
         body.append(f"  mu = (double)({de});")
         body.append("  if (c != c) mu = LCM_NAN;")
         body.append("  if (rv == -LCM_INF) mu = 0.0;")
@@ -473,7 +475,7 @@ class EgmKernels:
         body.append("    double2 es; lcm_bracket_slopes(RG[k], RG[k + 1], rv, rv1, mu, mu1, es.x, es.y);")
         body.append("    ES[k] = es;")
         body.append("  }")
-        body.append("  RV[k] = rv;")
+        body.append("  lcm_st_relaxed(RV + k, rv);")
         body.append("  RM[k] = mu;")
         body.append("}")
         for s in body:
