@@ -739,19 +739,26 @@ class RegimeKernels:
                     "nob": spec.actions[kob].size, "x0": x0, "g": g, "namax": namax}
         return None
 
+    def _ascending(self, action: str) -> bool:
+        values = np.asarray(next(a for a in self.spec.actions if a.name == action).grid.to_numpy(), dtype=np.float64)
+        return bool(np.all(np.diff(values) >= 0.0))
+
     def _budget_bound(self):
         """(action position, bound node, strict) of a constraint a <= b (or
         b >= a, or strict) in F, where `a` is the slowest continuous action --
         every action before it discrete, so that its index is the slowest
         part of the continuous-action index and, its grid being ascending, the
         feasible actions of a state form a prefix of the table -- and `b` reads
-        no action.  None if F has no such constraint."""
+        no action.  None if F has no such constraint, or the grid descends (a
+        logarithmic grid may)."""
         spec = self.spec
         names = [a.name for a in spec.actions]
         kc = next((k for k, a in enumerate(spec.actions) if a.kind == "continuous"), None)
         if kc is None:
             return None
         cname = names[kc]
+        if not self._ascending(cname):
+            return None
         F = ir.const(self.tr.F)
         stack = [F] if isinstance(F, ir.Expr) else []
         while stack:
@@ -944,7 +951,9 @@ class RegimeKernels:
         """The action-free side b of a constraint scan <= b (or <, or b >=
         scan) in F: the scan action's grid being ascending, the actions that
         meet it are a prefix of the grid.  None if F has no such
-        constraint."""
+        constraint, or the grid descends."""
+        if not self._ascending(scan):
+            return None
         F = ir.const(self.tr.F)
         stack = [F] if isinstance(F, ir.Expr) else []
         while stack:
