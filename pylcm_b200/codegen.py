@@ -2459,8 +2459,14 @@ class RegimeKernels:
 
         `fast` evaluates an action without branches, `call` with the
         zero-safe rule.  In double precision with a collapsed axis `fast`
-        reads the collapsed row, an ulp or so away from the bilinear read of
-        `call`: it only rules actions out, `call` decides."""
+        reads the collapsed row, whose coordinate K + M * action rounds
+        otherwise than the law as written in `call`: it only rules actions
+        out, by more than the cover `cov` of both coordinates' rounding (64
+        ulps of their terms' magnitudes, sA and sB nodes, times the largest
+        step of the values it reads, weights beyond the grid, xA and xB nodes
+        out, included), and `call` decides.  A row entry whose coordinate may
+        fall on either side of a node beside a value that is not finite is
+        NaN: nothing is ruled out there."""
         fp32 = self.precision == "fp32"
         ST = "float" if fp32 else "double"
         p, x = self._line, li["x"]
@@ -2528,6 +2534,12 @@ class RegimeKernels:
               "}"]
         if verify:
             b.append(f"if (threadIdx.x < {nrow}) gAbs[threadIdx.x] = 0;")
+            b.append("__syncthreads();")
+
+        def magnitude_b(action: str) -> str:  # of the terms of the collapsed coordinate, in nodes
+            return (f"(fabs((double)({li['B'][0]})) + fabs((double)C.a{ti}_{coll['cb']}) + "
+                    f"fabs((double)({li['B'][1]}) * {action})) * fabs((double)C.b{ti}_{coll['cb']})")
+
         if coll:
             cb = coll["cb"]
             b += [f"const int nB = C.n{ti}_{coll['posB']};",
@@ -2543,8 +2555,17 @@ class RegimeKernels:
             else:
                 b.append(f"  const {ST} va = blk[(i64)lB * nA + w], vb = blk[(i64)(lB + 1) * nA + w];")
             b += [f"  {ST} val = va + uB * (vb - va);",
-                  f"  if (!lcm_isfinite(val)) val = lcm_zs(({ST})1 - uB, va) + lcm_zs(uB, vb);",
-                  "  row[e] = val;",
+                  f"  if (!lcm_isfinite(val)) val = lcm_zs(({ST})1 - uB, va) + lcm_zs(uB, vb);"]
+            if verify:
+                nd = f"blk[(i64)w * nB + n]" if cb == 1 else f"blk[(i64)n * nA + w]"
+                b += [f"  if (fabs(cB - rint(cB)) <= 1.5e-14 * (1.0 + {magnitude_b('obg[ob]')})) {{",
+                      "    bool fin = true;",
+                      f"    for (int n = max(lB - 1, 0); n <= min(lB + 2, nB - 1); ++n) fin = fin && lcm_isfinite({nd});",
+                      "    if (!fin) val = lcm_lim<double>::nan();",
+                      "  }",
+                      "  const double big = fmax(lcm_isfinite(va) ? fabs(va) : 0.0, lcm_isfinite(vb) ? fabs(vb) : 0.0);",
+                      "  atomicMax(&gAbs[ob], __float_as_int(__double2float_ru(big * (1.0 + 2.0 * fmax(0.0, fmax(-cB, cB - (nB - 1)))))));"]
+            b += ["  row[e] = val;",
                   "}"]
         else:
             b += [f"const {ST}* src = C.ev{ti} + (i64)({li['key']}) * nA;",
@@ -2554,8 +2575,6 @@ class RegimeKernels:
               f"for (int e = threadIdx.x; e < {nrow} * nA; e += {B}) {{",
               "  const int lim = min(win, nA - e % nA);",
               f"  {ST} m = row[e], a = lcm_isfinite(m) ? {fabs_}(m) : ({ST})0;"]
-        if verify:
-            b.append("  atomicMax(&gAbs[e / nA], __float_as_int(__double2float_ru(a)));")
         b += ["  #pragma unroll 4\n  for (int k = 1; k < lim; ++k) {",
               f"    const {ST} v = row[e + k];",
               "    m = lcm_nanmax(m, v);",
@@ -2587,15 +2606,22 @@ class RegimeKernels:
                   f"const {ST}* rrow = row + obi * nA; const float2* mrow = mw + obi * nA;"]
         else:
             c.append(f"const {ST}* rrow = row; const float2* mrow = mw;")
-        if verify:
-            c.append(f"const double babs = (double)beta_b * (double)__int_as_float(gAbs[obi]);")
         c.append("const float4* grp = gI + o_ * gpc;")
         c.append("float gK = gK0, gE = gE0 + fabsf(gM) * fmaxf(fabsf(grp[0].y), fabsf(grp[gpc - 1].z));")
         for nm in others:
             c.append(f"{{ const float v = ((float)({li['co'][nm]}) * {Bs}) * (float)ltab[jb0 * {nf} + {li['avf'][nm]}]; "
                      "gK += v; gE += fabsf(v); }")
-        c += ["gE = 0.02f + 4e-6f * gE;  // cover of the coordinate's rounding in the search",
-              "const float gTop = (float)(nA - 1);"]
+        c.append("const float gTop = (float)(nA - 1);")
+        if verify:
+            c += ["// cover of the collapsed read against the bilinear one",
+                  "const float e0_ = gM * grp[0].y + gK, e1_ = gM * grp[gpc - 1].z + gK;",
+                  "const double sA = (double)gE, xA = fmax(0.0, (double)fmaxf(-fminf(e0_, e1_), fmaxf(e0_, e1_) - gTop) + 0.02 + 4e-6 * sA);",
+                  f"const double obv = lcm_wp<const double>(it, {self.W_AGRID + coll['kob']})[obi];",
+                  f"const double sB = {magnitude_b('obv')};",
+                  "const double cov = (double)beta_b * (double)__int_as_float(gAbs[obi]) * "
+                  "(1e-13 + 1.5e-14 * ((1.0 + 2.0 * xA) * (1.0 + 2.0 * sB) + 2.0 * sA));",
+                  "const float covf = __double2float_ru(cov);"]
+        c.append("gE = 0.02f + 4e-6f * gE;  // cover of the coordinate's rounding in the search")
 
         def load(j: str) -> list[str]:
             if nf == 2:
@@ -2633,7 +2659,7 @@ class RegimeKernels:
             c.append(f"    const {ST} b1 = __shfl_xor_sync(0xffffffffu, p1, w), b2 = __shfl_xor_sync(0xffffffffu, p2, w);")
             c.append(f"    p2 = {fmax_}({fmin_}(p1, b1), {fmax_}(p2, b2)); p1 = {fmax_}(p1, b1);")
             c.append("  }")
-        p_ = "p2" if fp32 else ("p1 - 1e-13 * (fabs(p1) + babs)" if verify else "p1")
+        p_ = "p2" if fp32 else ("p1 - (1e-13 * fabs(p1) + cov)" if verify else "p1")
         c.append(f"  if (p1 > {ninf}) thr = {fmax_}(thr, {p_});")
         c.append("}")
         # group tests (NT at a time, branch-free, so that their chains overlap)
@@ -2664,7 +2690,8 @@ class RegimeKernels:
               "    }",
               f"    #pragma unroll\n    for (int k = 0; k < {NT}; ++k) {{",
               f"      const int b_ = b0 + {LANES} * k;",
-              "      const bool skip = in_[k] && tu[k] + beta_b * tm[k].x + 4.8e-7f * (fabsf(tu[k]) + beta_b * tm[k].y) < th;",
+              "      const bool skip = in_[k] && tu[k] + beta_b * tm[k].x + 4.8e-7f * (fabsf(tu[k]) + beta_b * tm[k].y)"
+              + (" + covf" if verify else "") + " < th;",
               f"      if (!skip && b_ < gc && (g0 + b_) * {G} < jfe) need |= 1u << b_;",
               "    }",
               "  }"]
@@ -2691,9 +2718,9 @@ class RegimeKernels:
               "        }"]
         if verify:
             c += [f"        const double cut = {cut};",
-                  "        if (okm && (bad || !(qm + 1e-13 * (fabs(qm) + babs) < cut))) {",
+                  "        if (okm && (bad || !(qm + (1e-13 * fabs(qm) + cov) < cut))) {",
                   f"          for (int k = 0; k < {NB}; ++k) {{",
-                  "            if (!((okm >> k) & 1u) || qv[k] + 1e-13 * (fabs(qv[k]) + babs) < cut) continue;",
+                  "            if (!((okm >> k) & 1u) || qv[k] + (1e-13 * fabs(qv[k]) + cov) < cut) continue;",
                   f"            const int j = jb0 + (i0 + tb + {LANES} * k) * gS;"]
             c += ["            " + s for s in ev]
             c += [f"            if ({call}) best[0].put(q, ad * n_ac + j);",
