@@ -187,7 +187,7 @@ class SolveEngine:
         self.specs = model.regime_specs
         self._kernels: dict[tuple, RegimeKernels] = {}
         self._bases: dict[tuple, RegimeKernels] = {}  # before the batch's launch shape is chosen
-        self._by_batch: dict[tuple, RegimeKernels] = {}  # (regime, targets, instances)
+        self._by_batch: dict[tuple, RegimeKernels] = {}  # (regime, targets, instances, shape asked for)
         self._traces: dict[tuple, TracedRegime] = {}
         self._spare: SolvePlan | None = None  # the plan of a finished one-instance call
         self._targets: dict[tuple, tuple] = {}
@@ -208,7 +208,8 @@ class SolveEngine:
         return self.configs.get(spec.name) or default_config(spec, self.precision, n_items)
 
     def kernels(self, spec: RegimeSpec, targets: tuple[str, ...], params, n_items: int = 1) -> RegimeKernels:
-        rk = self._by_batch.get((spec.name, targets, n_items))
+        asked = (spec.name, targets, n_items, self.configs.get(spec.name))  # `configs` may change between calls
+        rk = self._by_batch.get(asked)
         if rk is not None:
             return rk
         cfg = self.config_for(spec, n_items)
@@ -228,7 +229,7 @@ class SolveEngine:
             rk.src = src
             rk.key = "lcm_" + hashlib.sha1(src.encode()).hexdigest()[:24]
             self._kernels[key] = rk
-        self._by_batch[(spec.name, targets, n_items)] = rk
+        self._by_batch[asked] = rk
         return rk
 
     def egm_kernels(self, spec: RegimeSpec, targets: tuple[str, ...], params):
