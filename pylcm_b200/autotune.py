@@ -10,7 +10,9 @@ batch-size bucket, so tuning runs once per (model structure, batch bucket).
 The candidate set is built around the occupancy heuristic of
 ``engine.default_config``: lanes in {L/2, L, 2L} (L the heuristic), states per
 thread in {1, 2} (and 4 in the single-precision search), block in {128, 256},
-action chunk in {256, 512}.
+action chunk in {256, 512}.  The shape that a batch gets without tuning is one
+of them, and where that is the full search (``RegimeKernels.line_config``) so
+are the others.
 
 A candidate that NVRTC cannot compile, or whose launch the driver refuses
 (resources), is skipped.  Any other failure -- in particular an error left
@@ -22,6 +24,7 @@ Used by ``BatchSolver(..., autotune=True)`` and ``Server(..., autotune=True)``.
 
 from __future__ import annotations
 
+import dataclasses
 import hashlib
 import itertools
 import json
@@ -64,6 +67,14 @@ def candidates(spec, precision: str, n_items: int) -> list[LaunchConfig]:
     return out
 
 
+def regime_candidates(eng: SolveEngine, spec, params, n_items: int) -> list[LaunchConfig]:
+    """`candidates` of a regime at this batch size, in the search form that it
+    takes without tuning, after the shape that it takes without tuning."""
+    own = eng.kernels(spec, eng.targets_at(spec, min(spec.active_periods)), params, n_items).cfg
+    rest = [dataclasses.replace(c, prune=own.prune) for c in candidates(spec, eng.precision, n_items)]
+    return [own, *(c for c in rest if c != own)]
+
+
 def _skippable(e: Exception) -> bool:
     """A candidate failure that leaves the context usable: NVRTC rejected
     the source (LCMX_ERR_COMPILE) or the driver refused the launch
@@ -92,7 +103,8 @@ def _time_regime(model, precision: str, params_list, spec, cfg: LaunchConfig, re
         b = torch.cuda.Event(enable_timing=True)
         a.record(s)
         l.module.module.bellman_step(
-            l.kernel, ib + 8 * l.item_off, pb + 4 * l.prefix_off, l.n_items, l.n_tiles, l.block, l.smem, s.cuda_stream
+            l.kernel, ib + 8 * l.item_off, pb + 4 * l.prefix_off, l.n_items, l.n_tiles, l.block, l.smem, s.cuda_stream,
+            grid=l.grid,
         )
         b.record(s)
         torch.cuda.synchronize()
@@ -121,7 +133,7 @@ def tune(model, precision: str, params_list, regimes: list[str] | None = None, v
             out[spec.name] = LaunchConfig(**hit)
             continue
         results = []
-        for cfg in candidates(spec, precision, n):
+        for cfg in regime_candidates(eng, spec, params_list[0], n):
             try:
                 t = _time_regime(model, precision, params_list, spec, cfg)
             except Exception as e:
@@ -140,7 +152,8 @@ def tune(model, precision: str, params_list, regimes: list[str] | None = None, v
         results.sort(key=lambda r: r[0])
         best = results[0][1]
         out[spec.name] = best
-        cache[key] = {"block": best.block, "lanes": best.lanes, "chunk": best.chunk, "sb": best.sb, "min_blocks": best.min_blocks}
+        cache[key] = {"block": best.block, "lanes": best.lanes, "chunk": best.chunk, "sb": best.sb,
+                      "min_blocks": best.min_blocks, "prune": best.prune}
         CACHE.parent.mkdir(parents=True, exist_ok=True)
         tmp = CACHE.with_suffix(".tmp")
         tmp.write_text(json.dumps(cache, indent=1))

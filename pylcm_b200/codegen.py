@@ -478,6 +478,10 @@ class LaunchConfig:
     # single-precision search: read a target with two continuous axes from
     # per-tile collapsed rows where eligible (see RegimeKernels._collapse_info)
     collapse: bool = True
+    # continuous axes of a target that the line form takes: 1 leaves a regime
+    # with two to the search by collapsed rows (the faster one there over long
+    # horizons, see RegimeKernels.line_config)
+    line_axes: int = 2
 
     @property
     def states_per_tile(self) -> int:
@@ -926,6 +930,8 @@ class RegimeKernels:
                 pos, ca = t.cont_pos[0], 0
                 if two:
                     coll = self._collapse_info(ti, t)
+                    if coll is not None and self.cfg.line_axes < 2:
+                        return None
                     if coll is None or coll["ob"] == scan or (line is not None and coll["line"] != line):
                         continue
                     pos, ca = coll["posA"], coll["ca"]

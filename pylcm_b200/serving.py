@@ -181,6 +181,12 @@ class Server:
     buffers of the jobs in flight.
     """
 
+    # of a family's regimes unless tuned or given: jobs of tens of requests, 2
+    # lanes x 2 states per thread (line form: one thread per state, 2 strips).
+    # Regimes with two continuous states keep the search by collapsed rows: NaN
+    # values make the line form the slower one over long horizons
+    SHAPE = LaunchConfig(block=256, lanes=2, chunk=512, sb=2, line_axes=1)
+
     def __init__(self, device: int = 0, precision: str = "fp32", max_batch: int = 32, n_streams: int = 4,
                  hbm_budget_bytes: int | None = None, configs: Mapping | None = None, pool_slots: int = 4,
                  autotune: bool = False) -> None:
@@ -235,8 +241,7 @@ class Server:
                 cfgs.update(self.configs.get(req.family, {}))
                 for s in req.model.regime_specs:
                     if s.name not in cfgs:
-                        # jobs of tens of requests: 2 lanes x 2 states per thread
-                        cfgs[s.name] = LaunchConfig(block=256, lanes=2, chunk=512, sb=2)
+                        cfgs[s.name] = self.SHAPE
                 self._family_cfg[req.family] = cfgs
             eng = SolveEngine(req.model, self.precision, configs=cfgs, device=self.device)
             self._engines[req.key] = eng
