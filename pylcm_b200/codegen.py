@@ -512,6 +512,8 @@ class RegimeKernels:
         self._affine = self._affine_all if precision == "fp32" else {}
         self._groups = self._group_plan()
         self._line = self._line_plan()
+        if self._line is not None and not self._line_fits():
+            self._line = None
         tag_src = repr(
             (self.spec.name, [t.spec.name for t in self.targets], precision, dataclasses.astuple(cfg))
         )
@@ -953,6 +955,32 @@ class RegimeKernels:
                 "scan": scan, "kscan": [a.name for a in spec.actions].index(scan), "acts": acts,
                 "cacts": [a.name for a in cacts], "budget": self._scan_bound(scan)}
 
+    def _line_bytes(self, line: dict) -> int:
+        """Shared memory of the line form: the whole continuous-action table,
+        then the rows' windowed maxima and the rows."""
+        cols = self._boundaries()["A"]
+        value = 4 if self.precision == "fp32" else 8
+        n_ac = self.spec.n_actions // self.spec.n_discrete_actions
+        rows = max((x["coll"]["nob"] if x["coll"] else 1) * self.targets[ti].spec.states[x["pos"]].size
+                   for ti, x in line["targets"].items())
+        return ((n_ac + 3) // 4 * 4 * sum(value if n.dtype == "f" else 4 for n in cols)) + rows * (8 + value)
+
+    def _line_fits(self) -> bool:
+        """Do the model's grids fit the line form?  A kernel that finds at run
+        time that they do not walks every action in a shape made for skipping:
+        such regimes keep the search and the shape that they would have
+        without it (B200, three solved periods, line shape / this: 64
+        instances of 500 x 3000, single precision 11.8 / 10.8 ms, double 15.0 /
+        12.3; 16 of 9000 x 500, 7.7 / 6.9 and 10.0 / 8.0; 256 of 500 x 15, 0.72
+        / 0.63 and 0.50 / 0.43)."""
+        spec, p = self.spec, self._line
+        if spec.n_actions // spec.n_discrete_actions > self.LINE_MAX_ACTIONS or self._line_bytes(p) > self.LINE_MAX_SMEM:
+            return False
+        if any(x["coll"] for x in p["targets"].values()):
+            return True
+        short = any(self.targets[ti].spec.states[x["pos"]].size < 2 for ti, x in p["targets"].items())
+        return spec.actions[p["kscan"]].size >= 2 * self.LINE_GROUP and not short
+
     def _scan_bound(self, scan: str):
         """The action-free side b of a constraint scan <= b (or <, or b >=
         scan) in F: the scan action's grid being ascending, the actions that
@@ -1031,6 +1059,8 @@ class RegimeKernels:
         nline = spec.states[self._line["kline"]].size
         lines = spec.n_states // nline * n_items
         lanes = next((k for k, n in ((1, 60_000), (2, 30_000), (4, 12_000), (8, 6_000)) if total >= n), 16)
+        while lanes > self.LINE_GROUP and spec.actions[self._line["kscan"]].size < 2 * lanes:
+            lanes //= 2  # two groups at least (a group holds an action per thread)
         most = math.ceil(nline / (cfg.block // lanes))
         build = 0.35
 
@@ -1157,6 +1187,35 @@ class RegimeKernels:
                 roots.append(t.laws[t.spec.states[pos].name].expr)
         return [ir.const(r) for r in roots]
 
+    def _phase(self, n: ir.Expr) -> str:
+        dnames = {a.name for a in self.spec.actions if a.kind != "continuous"}
+        d = n.deps()
+        has_s = any(k == "state" for k, _ in d)
+        has_ac = any(k == "action" and nm not in dnames for k, nm in d)
+        has_ad = any(k == "action" and nm in dnames for k, nm in d)
+        if has_ac:
+            return "SA" if has_s else "A"
+        if has_s:
+            return "SD" if has_ad else "S"
+        return "D" if has_ad else "P"
+
+    def _boundaries(self) -> dict[str, list]:
+        """Boundary nodes the inner loop of kernel (a) consumes, by phase."""
+        bnd: dict[str, list] = {k: [] for k in ("P", "D", "S", "SD", "A")}
+        seen: set[int] = set()
+        stack = [r for r in self._roots() if isinstance(r, ir.Expr)]
+        while stack:
+            n = stack.pop()
+            if id(n) in seen or n.op == "const":
+                continue
+            seen.add(id(n))
+            ph = self._phase(n)
+            if ph != "SA":
+                bnd[ph].append(n)
+                continue
+            stack.extend(a for a in n.args if isinstance(a, ir.Expr))
+        return bnd
+
     def _bellman_source(self) -> str:
         """Kernel (a0) (action table) and kernel (a) (Bellman step) for this regime.
 
@@ -1182,38 +1241,12 @@ class RegimeKernels:
         taste = spec.taste_shocks
         dacts = [a for a in spec.actions if a.kind != "continuous"]
         cacts = [a for a in spec.actions if a.kind == "continuous"]
-        dnames = {a.name for a in dacts}
         ND = spec.n_discrete_actions
 
-        def phase(n: ir.Expr) -> str:
-            d = n.deps()
-            has_s = any(k == "state" for k, _ in d)
-            has_ac = any(k == "action" and nm not in dnames for k, nm in d)
-            has_ad = any(k == "action" and nm in dnames for k, nm in d)
-            if has_ac:
-                return "SA" if has_s else "A"
-            if has_s:
-                return "SD" if has_ad else "S"
-            return "D" if has_ad else "P"
-
-        roots = self._roots()
         det = self.tr.regime_id is not None and bool(self.targets)
-        rid_phase = phase(self.tr.regime_id) if det else None
+        rid_phase = self._phase(self.tr.regime_id) if det else None
         unswitch = det and rid_phase in ("P", "D")
-        # boundary nodes the inner loop consumes, by phase
-        bnd: dict[str, list] = {k: [] for k in ("P", "D", "S", "SD", "A")}
-        seen: set[int] = set()
-        stack = [r for r in roots if isinstance(r, ir.Expr)]
-        while stack:
-            n = stack.pop()
-            if id(n) in seen or n.op == "const":
-                continue
-            seen.add(id(n))
-            ph = phase(n)
-            if ph != "SA":
-                bnd[ph].append(n)
-                continue
-            stack.extend(a for a in n.args if isinstance(a, ir.Expr))
+        bnd = self._boundaries()
         bP, bD, bS, bSD, bA = bnd["P"], bnd["D"], bnd["S"], bnd["SD"], bnd["A"]
         if unswitch and id(self.tr.regime_id) not in {id(x) for x in bP + bD}:
             (bP if rid_phase == "P" else bD).append(self.tr.regime_id)
@@ -1254,17 +1287,8 @@ class RegimeKernels:
         rows_bytes = max((2 * c["nob"] * c["namax"] * 4 for c in cinfo.values()), default=0)
         TB = 4 if fp32 else 8  # bytes of a search value
         if line is not None:
-            # the line form lays its shared memory out at run time: the whole
-            # continuous-action table, then the rows' windowed maxima and the
-            # rows
-            n_ac = spec.n_actions // ND
-            tab = (n_ac + 3) // 4 * 4 * (nf * TB + ni * 4)
-            rows_bytes = max((x["coll"]["nob"] if x["coll"] else 1) * self.targets[ti].spec.states[x["pos"]].size
-                             for ti, x in line["targets"].items()) * (12 if fp32 else 16)
-            line_bytes = tab + rows_bytes
-            if n_ac > self.LINE_MAX_ACTIONS or line_bytes > self.LINE_MAX_SMEM:
-                line_bytes = 0  # the kernel sees the shortage and runs the plain loop
-            rows_bytes = max(0, line_bytes - (NF * CH * TB + NI * CH * 4))
+            # the line form lays its shared memory out at run time
+            rows_bytes = max(0, self._line_bytes(line) - (NF * CH * TB + NI * CH * 4))
 
         L: list[str] = []
         ap = L.append
