@@ -1243,7 +1243,12 @@ class SolvePlan:
     # Most of these launches leave the GPU mostly idle (7 to 14 us each at
     # 1.5 us of work).  The tensor-core expectations stay in one branch: a CTA
     # holds tensor memory, and another launch's CTAs would wait for it.
-    MAX_LANES = 8
+    # Five branches: instantiating the graph takes longer with each (256 x 500
+    # x 500, 40 periods, single precision, 1 / 3 / 4 / 5 / 8 branches: 0.8 / 5.4
+    # / 13 / 23 / 87 ms, once per solver) and a replay gains nothing beyond
+    # (32.6 / 32.5 / 31.5 / 30.0 / 30.9 ms; 48 x 333 x 401, 12 periods, double:
+    # 2.79 / 2.75 / 2.18 / 2.21 / 2.35).
+    MAX_LANES = 5
 
     def _lanes(self) -> list[int]:
         """The branch (0: the capturing stream) of every launch: the step's
