@@ -514,10 +514,13 @@ class RegimeKernels:
         self._line = self._line_plan()
         if self._line is not None and not self._line_fits():
             self._line = None
-        tag_src = repr(
-            (self.spec.name, [t.spec.name for t in self.targets], precision, dataclasses.astuple(cfg))
-        )
-        self.tag = self.spec.name.replace("-", "_") + "_" + hashlib.sha1(tag_src.encode()).hexdigest()[:8]
+        # kernel (a) carries the launch shape in its tag; the other kernels are
+        # the same for every shape
+        what = (self.spec.name, [t.spec.name for t in self.targets], precision)
+        shape = cfg if self._line is None else dataclasses.replace(cfg, sb=1)  # (strips are an item word)
+        name = self.spec.name.replace("-", "_") + "_"
+        self.tag = name + hashlib.sha1(repr((*what, dataclasses.astuple(shape))).encode()).hexdigest()[:8]
+        self.rtag = name + hashlib.sha1(repr(what).encode()).hexdigest()[:8]
 
     # -------------------------------------------------------------- layout
     def _layout(self) -> None:
@@ -543,6 +546,7 @@ class RegimeKernels:
         self.W_AGRID = take(len(spec.actions))
         self.W_TASTE = take()
         self.W_ATAB = take()  # global action table (kernel a0 output) of this item
+        self.W_STRIPS = take()  # line form: strips of a line per CTA
         for t in self.targets:
             if t.unreachable:
                 continue
@@ -562,10 +566,40 @@ class RegimeKernels:
 
     # -------------------------------------------------------------- source
     def source(self) -> str:
-        parts = [device_header(), _EXTRA_DEVICE, self._bellman_source()]
+        """Every kernel in one text."""
+        return "\n".join(text for _, text in self._sections())
+
+    def sources(self) -> tuple[str, str]:
+        """(kernel (a), the other kernels) as modules of their own: the second
+        does not name the launch shape, so that a batch size that takes another
+        shape compiles kernel (a) alone (1.4 of 2.5 s of NVRTC for the
+        stochastic model's working regime, 0.6 of 2.7 for the human-capital
+        model's)."""
+        sections = self._sections()
+        a = "\n".join(text for part, text in sections if part in ("both", "a"))
+        rest = "\n".join(text for part, text in sections if part in ("both", "rest"))
+        return a, rest.replace(self.tag, self.rtag)
+
+    def _sections(self) -> list[tuple[str, str]]:
+        """The generated text in pieces: of kernel (a) ("a"), of the other
+        kernels ("rest") and of both."""
+        out = self.__dict__.get("_text")
+        if out is not None:
+            return out
+        out = [("both", device_header())]
         tc = [t for t in self.targets if self.tc_ok(t)]
         if tc:
-            parts.insert(1, tc_header())
+            out.append(("rest", tc_header()))
+        out.append(("both", _EXTRA_DEVICE))
+        part, lines = "both", []
+        for ln in self._bellman_source():
+            if ln.startswith("//@"):
+                out.append((part, "\n".join(lines)))
+                part, lines = ln[3:], []
+            else:
+                lines.append(ln)
+        out.append((part, "\n".join(lines)))
+        parts: list[str] = []
         for t in self.targets:
             if not t.scalar and (t.needs_contraction or self.precision == "fp32"):
                 parts.append(self._expect_source(t))
@@ -575,7 +609,9 @@ class RegimeKernels:
             parts.append(f'extern "C" __global__ void __launch_bounds__(256) {self.stats_name()}('
                          "const i64* __restrict__ items, const int* __restrict__ tile_prefix, int n_items, "
                          "int n_tiles) {\n  lcm_tile_stats2(items, tile_prefix, n_items, n_tiles);\n}")
-        return "\n".join(parts)
+        out += [("rest", x) for x in parts]
+        self._text = out
+        return out
 
     def e_words_for(self, t: TargetPlan) -> int:
         return 9 + len(t.spec.states)
@@ -584,10 +620,10 @@ class RegimeKernels:
         return f"lcm_bellman_{self.tag}"
 
     def atab_name(self) -> str:
-        return f"lcm_atab_{self.tag}"
+        return f"lcm_atab_{self.rtag}"
 
     def expect_name(self, t: TargetPlan) -> str:
-        return f"lcm_expect_{self.tag}_{t.spec.name}"
+        return f"lcm_expect_{self.rtag}_{t.spec.name}"
 
     # ..................................................................
     def _sim_extrapolated_expectation(self, ti, t, T, E, blend, proc_names, dn, mk) -> list[str]:
@@ -1119,7 +1155,7 @@ class RegimeKernels:
         return len(g["axes"][ti])
 
     def stats_name(self) -> str:
-        return f"lcm_tile_stats_{self.tag}"
+        return f"lcm_tile_stats_{self.rtag}"
 
     def inner_flops(self) -> dict:
         """Floating-point operations of one (state, action) evaluation of
@@ -1216,8 +1252,10 @@ class RegimeKernels:
             stack.extend(a for a in n.args if isinstance(a, ir.Expr))
         return bnd
 
-    def _bellman_source(self) -> str:
-        """Kernel (a0) (action table) and kernel (a) (Bellman step) for this regime.
+    def _bellman_source(self) -> list[str]:
+        """Kernel (a0) (action table), kernel (a) (Bellman step) and kernel (d)
+        (simulation) of this regime: lines, a line "//@part" before each piece
+        of another part (see `_sections`).
 
         Loop structure of kernel (a), per tile of states:
 
@@ -1269,8 +1307,8 @@ class RegimeKernels:
             LANES, SB = self.line_lanes, 1
         elif self._groups:
             CH = max(CH, self.GROUP_MAX_CHUNK)  # group skipping holds the whole table
-        SPT = cfg.states_per_tile if line is None else self.line_tile
         SPB = B // LANES
+        SPT = cfg.states_per_tile if line is None else f"(strips * {SPB})"
         dstates = [a for a in spec.states if a.kind != "continuous"]
         NDS = max(len(dstates), 1)
         nP, nD, nS, nSD = (max(len(x), 1) for x in (bP, bD, bS, bSD))
@@ -1334,6 +1372,7 @@ class RegimeKernels:
 
         # ----------------------------------------------------------------
         # accessors of the continuous-action table
+        ap("//@a")
         ap(
             f"template <typename T> struct AFTab_{self.tag} {{ const {TT}* tabf; const int* tabi; int j;\n"
             f"  __device__ __forceinline__ T F(int f) const {{ return (T)tabf[f * {CH} + j]; }}\n"
@@ -1590,6 +1629,7 @@ class RegimeKernels:
                 ap("  " + s_)
             ap("  return ok_;\n}")
 
+        ap("//@rest")
         ap(
             f"template <typename T, typename E, typename AFN>\n"
             f"__device__ __forceinline__ bool lcm_simsa_{self.tag}(const Ctx_{self.tag}<T, E>& C, "
@@ -1642,6 +1682,7 @@ class RegimeKernels:
         # ----------------------------------------------------------------
         # kernel (a)
         SA = f"lcm_sa{{}}_{self.tag}"
+        ap("//@a")
         ap(
             f'extern "C" __global__ void __launch_bounds__({B}{", " + str(cfg.min_blocks) if cfg.min_blocks else ""}) '
             f"{self.bellman_name()}(const i64* __restrict__ items, const int* __restrict__ tile_prefix, int n_items, int n_tiles) {{"
@@ -1666,7 +1707,8 @@ class RegimeKernels:
             ap(f"    const int sbase = (tile - tile_prefix[item]) * {SPT} + (int)threadIdx.x / {LANES};")
         else:
             ap(f"    const int nLine = lcm_wi(it, {self.W_SSIZE + line['kline']});")
-            ap(f"    const int ppl = (nLine + {SPT - 1}) / {SPT};  // parts of a line")
+            ap(f"    const int strips = lcm_wi(it, {self.W_STRIPS});")
+            ap(f"    const int ppl = (nLine + {SPT} - 1) / {SPT};  // parts of a line")
             ap("    const int line_id = (tile - tile_prefix[item]) / ppl;")
             ap(f"    const int part0 = (tile - tile_prefix[item] - line_id * ppl) * {SPT};")
             ap('    unsigned dyn_smem; asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(dyn_smem));')
@@ -1680,7 +1722,7 @@ class RegimeKernels:
         if not bP:
             ap("    PVd[0] = 0.0;")
         if line is not None:
-            ap(f"    for (int strip = 0; strip < {cfg.sb}; ++strip) {{")
+            ap("    for (int strip = 0; strip < strips; ++strip) {")
             ap(f"    const int pos0 = part0 + strip * {SPB};")
             ap("    if (pos0 >= nLine) break;  // uniform over the CTA")
         ap(f"    int SI[{SB}][{NDS}]; double SV[{SB}][{nS}]; bool act[{SB}]; int sidx[{SB}];")
@@ -2399,6 +2441,7 @@ class RegimeKernels:
 
         # ----------------------------------------------------------------
         # kernel (a0): continuous-action-only sub-expressions, one thread per action
+        ap("//@rest")
         ap(f"// ---- regime {spec.name}: action table (kernel a0)")
         ap(
             f'extern "C" __global__ void __launch_bounds__(256) {self.atab_name()}('
@@ -2440,8 +2483,7 @@ class RegimeKernels:
         ap("    }")
         ap("  }")
         ap("}")
-        L += self._sim_kernel(locals())
-        return "\n".join(L)
+        return L + self._sim_kernel(locals())
 
     def _line_prefix_lines(self, bP: list, bS: list, ST: str) -> list[str]:
         """Per state: `jfe`, the number of scan-action grid points that can
@@ -2816,7 +2858,7 @@ class RegimeKernels:
         self.sim_n_slots = q
 
     def sim_name(self) -> str:
-        return f"lcm_sim_{self.tag}"
+        return f"lcm_sim_{self.rtag}"
 
     def _sim_kernel(self, env: dict) -> list[str]:
         """Kernel (d): one simulated period of this regime for every subject in it.
@@ -3228,7 +3270,7 @@ class RegimeKernels:
                 and not t.det_pos and t.J <= self.TC_MAX_J and t.K <= self.TC_MAX_K)
 
     def expect_tc_name(self, t: TargetPlan) -> str:
-        return f"lcm_expect_tc_{self.tag}_{t.spec.name}"
+        return f"lcm_expect_tc_{self.rtag}_{t.spec.name}"
 
     @staticmethod
     def tc_shape(K: int, J: int) -> dict:

@@ -262,12 +262,16 @@ class SolveEngine:
         return vk
 
     def module(self, rk: RegimeKernels):
-        from pylcm_b200.runtime import get_context
+        from pylcm_b200.runtime import RegimeModule, get_context
 
         mod = getattr(rk, "module", None)
         if mod is None:
             ctx = get_context(self.device)
-            mod = ctx.compile(rk.src, rk.key)
+            if isinstance(rk, RegimeKernels):
+                a, rest = (ctx.compile(x, "lcm_" + hashlib.sha1(x.encode()).hexdigest()[:24]) for x in rk.sources())
+                mod = RegimeModule(rk.bellman_name(), a, rest)
+            else:
+                mod = ctx.compile(rk.src, rk.key)
             rk.module = mod
         return mod
 
@@ -608,6 +612,7 @@ class SolvePlan:
             r[rk.W_AGE] = _f2w(age)
             r[rk.W_NSTATES] = s.n_states
             r[rk.W_NACT] = s.n_actions
+            r[rk.W_STRIPS] = rk.cfg.sb
             for k, ax in enumerate(s.states):
                 r[rk.W_SSIZE + k] = ax.size
                 g = self.sgrid[s.name][k]

@@ -261,6 +261,30 @@ class Module:
         self.ctx.check(self.ctx.lib.lcmx_egm_step(self.h, kernel.encode(), ctypes.byref(a), stream))
 
 
+class RegimeModule:
+    """The two modules of a regime's generated kernels: kernel (a), compiled per
+    launch shape, and the others, which every shape shares."""
+
+    def __init__(self, bellman: str, a: Module, rest: Module) -> None:
+        self.bellman, self.a, self.rest = bellman, a, rest
+
+    def of(self, kernel: str) -> Module:
+        return self.a if kernel == self.bellman else self.rest
+
+    def prepared(self, kind: str, kernel: str, *args, **kwargs) -> "PreparedLaunch":
+        return self.of(kernel).prepared(kind, kernel, *args, **kwargs)
+
+    def bellman_step(self, kernel: str, *args, **kwargs) -> None:
+        self.of(kernel).bellman_step(kernel, *args, **kwargs)
+
+    def occupancy(self, kernel: str, block: int, smem: int) -> int:
+        return self.of(kernel).occupancy(kernel, block, smem)
+
+    def status(self, reset: bool = True) -> int:
+        """Of the tensor-core expectation (see Module.status)."""
+        return self.rest.status(reset)
+
+
 @contextlib.contextmanager
 def side_streams(ctx: Context, n: int):
     """`n` streams of nobody else's (torch's come from a shared pool), as torch
