@@ -463,6 +463,9 @@ def _target_plan(tr: TracedRegime, tgt: RegimeSpec) -> TargetPlan:
     return TargetPlan(tgt, False, prob, stoch, det, cont, key_vars, laws)
 
 
+SM_COUNT = 148  # of the B200
+
+
 @dataclasses.dataclass(frozen=True)
 class LaunchConfig:
     block: int = 256
@@ -1101,7 +1104,7 @@ class RegimeKernels:
         build = 0.35
 
         def cost(k: int) -> float:
-            return math.ceil(lines * math.ceil(most / k) / (2 * 148)) * (k + build)
+            return math.ceil(lines * math.ceil(most / k) / (2 * SM_COUNT)) * (k + build)
 
         strips = min((k for k in (1, 2, 4) if k <= max(1, most)), key=cost)
         return dataclasses.replace(cfg, lanes=2 * lanes, sb=strips)
@@ -1727,7 +1730,7 @@ class RegimeKernels:
             ap("    if (pos0 >= nLine) break;  // uniform over the CTA")
         ap(f"    int SI[{SB}][{NDS}]; double SV[{SB}][{nS}]; bool act[{SB}]; int sidx[{SB}];")
         if line is not None:
-            cinfo_rows, cinfo = cinfo, {}  # the rows are read by the line form only
+            cinfo = {}  # the rows are read by the line form only
         kline = next(iter(cinfo.values()))["kline"] if cinfo else -1
         if cinfo:
             # states walked with the line state fastest (a tile then covers at

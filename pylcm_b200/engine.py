@@ -28,7 +28,7 @@ from typing import Any, Sequence
 
 import numpy as np
 
-from pylcm_b200.codegen import LaunchConfig, RegimeKernels
+from pylcm_b200.codegen import SM_COUNT, LaunchConfig, RegimeKernels
 from pylcm_b200.exceptions import ModelInitializationError
 from pylcm_b200.runtime import bundle
 from pylcm_b200.egm import is_egm
@@ -130,7 +130,6 @@ class _Records:
         )
 
 
-SM_COUNT = 148
 # grid of launches whose tiles differ in work (see lcmx_launch_args): measured
 # on the B200, grid stride / one CTA per tile: DC-EGM continuation of 12 x 777
 # points 253 / 175 us, of 32 x 2000 (18 tiles per resident CTA) 614 / 634;

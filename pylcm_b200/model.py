@@ -102,6 +102,12 @@ class Model:
         double precision.  With ``return_policy=True`` a mapping of flat argmax
         action indices follows V in the returned tuple.  Unknown keywords raise
         ``TypeError``.
+
+        The host arrays of one regime (values, and policies) are slices of one
+        array, copied from the device at once: a caller who keeps one period's
+        keeps the regime's other periods in memory too.  ``V.copy()`` keeps a
+        period alone.  With ``return_device=True`` the device tensors of all
+        periods share a buffer in the same way.
         """
         _check_compat_kwargs(max_compilation_workers, log_path, log_keep_n_latest)
         from pylcm_b200.validation import validate_transitions

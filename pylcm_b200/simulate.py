@@ -28,7 +28,7 @@ from typing import Mapping
 
 import numpy as np
 
-from pylcm_b200.engine import UNEVEN
+from pylcm_b200.engine import SM_COUNT, UNEVEN
 from pylcm_b200.exceptions import InvalidInitialConditionsError, InvalidParamsError
 from pylcm_b200.grids import DiscreteGrid
 from pylcm_b200.runtime import bundle
@@ -183,11 +183,11 @@ def jax_key_chain(model, params, seed: int) -> dict:
 
 def subjects_per_warp(total: int) -> int:
     """Subjects a warp of kernel (d) takes in turn: a power of two up to 32
-    that leaves the GPU (148 SMs, 16 resident warps each at the kernel's 128
+    that leaves the GPU (16 resident warps per SM at the kernel's 128
     registers) about four waves of warps, so that small simulations still fill
     it and large ones draw for 32 subjects at once."""
     spw = 1
-    while spw < 32 and 2 * spw * 4 * 148 * 16 <= total:
+    while spw < 32 and 2 * spw * 4 * SM_COUNT * 16 <= total:
         spw *= 2
     return spw
 
