@@ -3283,7 +3283,7 @@ class RegimeKernels:
         NP = (K + 15) // 16 * 16
         ncol = 32 if NP <= 32 else 64 if NP <= 64 else 128 if NP <= 128 else 256
         dyn = 2 * 128 * JP * 4 + 2 * NP * JP * 4 + 128
-        static = K * J * 8 + K * 20 + 8 + 4 + 4 + 64
+        static = K * J * 8 + K * 4  # weights and row scales, the least of every form of the kernel
         # at most 512 / ncol CTAs per SM so that every CTA's tensor-memory
         # allocation succeeds at once: pad the dynamic shared memory so that
         # no more CTAs fit (228 KB per SM, 1 KB reserved per CTA)
