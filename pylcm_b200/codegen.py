@@ -942,8 +942,8 @@ class RegimeKernels:
         `_collapse_info`), on linear grids, whose coordinate x = x0 + sum_k
         coef_k a_k is affine in the continuous actions."""
         spec, tr = self.spec, self.tr
-        if (not self.cfg.prune or spec.terminal or spec.taste_shocks or tr.regime_id is None or tr.beta is None
-                or not self.targets):
+        if (not self.cfg.prune or self.cfg.line_axes < 1 or spec.terminal or spec.taste_shocks or tr.regime_id is None
+                or tr.beta is None or not self.targets):
             return None
         cacts = [a for a in spec.actions if a.kind == "continuous"]
         cstates = [a.name for a in spec.states if a.kind == "continuous"]
@@ -1058,17 +1058,35 @@ class RegimeKernels:
 
     # (state, action) pairs of a batch from which the line form pays
     LINE_MIN_PAIRS = 16_000_000
+    # us of a launch (B200, fitted to 63 grids x 2 to 4 batch sizes x 5 numbers
+    # of threads, see line_config): (launch, build per 1000 nodes of the line,
+    # strip, strip per action / threads) and of the full search (launch, per
+    # million pairs; for double precision 0.75 of the fit, so that a close call
+    # stays with it, for single 1.08, where the search before the line form
+    # was slower still)
+    LINE_COST = {"fp32": (4.6, 7.5, 11.2, 0.039), "fp64": (8.9, 12.3, 8.3, 0.056)}
+    FULL_COST = {"fp32": (13.0, 2.8), "fp64": (12.3, 1.73)}
 
     def line_config(self, n_items: int) -> LaunchConfig:
         """The launch shape of kernel (a) for `n_items` instances where the
-        caller asks for none.
+        caller asks for none: the line form's or the full search's, by what
+        either costs.
 
         Small batches: the full search, whose threads per state fill the GPU
         without the line form's per-CTA set-up (B200, milliseconds per solve
         batch, full search / line form: 3500 states x 1000 actions, double
-        precision, 0.475 / 0.525; 21,000 x 1000: 1.33 / 0.90).  The
-        single-precision search over one continuous action and one axis keeps
-        the line form at every size (3500 x 1000: 0.71 / 0.68).
+        precision, 0.475 / 0.525; 21,000 x 1000: 1.33 / 0.90).
+
+        Short lines, few actions: a CTA holds one line, so lines shorter than
+        its threads leave it mostly idle unless several threads share a state,
+        and its pilots and build cost as much as a few dozen actions (B200, us
+        per launch of 7-state shocks x 2 choices, full search / one thread per
+        state / the best number: wealth 62 x 105 actions x 219 instances,
+        double, 58 / 217 / 95; 62 x 400 x 288, 285 / 612 / 194; 800 x 30 x
+        298, 215 / 868 / 868; 500 x 400 x 36, 266 / 133 / 133; single, 62 x 60
+        x 384, 76 / 198 / 127; 500 x 400 x 36, 256 / 91 / 91).  Waves of CTAs x
+        (build + strips x (strip + actions / threads)) is within 18 % of the
+        launches measured.
 
         Two axes (collapsed rows): the full search.  The line form is up to
         twice as fast on large batches while the values are finite (1000 x 50 x
@@ -1078,35 +1096,42 @@ class RegimeKernels:
         instances of 1000 x 50 x 32 x 300, single precision) and 8.0 against
         4.0 (one, double).  On short lines, few lines or few scanned actions
         it loses at once (136 x 26 x 7 x 226, 128 / 206).  A launch shape that
-        is asked for (`configs`) takes it as before.
-
-        Threads per state: one, or more while the states do not fill the GPU
-        (21,000 states: 1 / 2 / 4 threads 1.34 / 0.95 / 0.90 ms; 70,000:
-        1.55 / 1.63 / 1.77).  Strips per CTA: a CTA that walks the whole line
-        builds its rows once, more CTAs fill the last wave better; the cheaper
-        of the two by waves x (strips + build), the build worth a third of a
-        strip (280 lines of 500: 2 strips 2.18, 1 strip 2.70 ms; 140 lines:
-        1.82, 1.55)."""
+        is asked for (`configs`) takes it as before."""
         cfg, spec = self.cfg, self.spec
         if self._line is None:
             return cfg
-        total = spec.n_states * n_items
+        full = dataclasses.replace(cfg, prune=False)
+        pairs = spec.n_states * n_items * spec.n_actions
         one = len(self._line["cacts"]) == 1
         two = any(x["coll"] for x in self._line["targets"].values())
-        if two or (total * spec.n_actions < self.LINE_MIN_PAIRS and not (one and self.precision == "fp32")):
-            return dataclasses.replace(cfg, prune=False)
+        if two or (pairs < self.LINE_MIN_PAIRS and not (one and self.precision == "fp32")):
+            return full
         nline = spec.states[self._line["kline"]].size
+        scan = spec.actions[self._line["kscan"]].size
         lines = spec.n_states // nline * n_items
-        lanes = next((k for k, n in ((1, 60_000), (2, 30_000), (4, 12_000), (8, 6_000)) if total >= n), 16)
-        while lanes > self.LINE_GROUP and spec.actions[self._line["kscan"]].size < 2 * lanes:
-            lanes //= 2  # two groups at least (a group holds an action per thread)
-        most = math.ceil(nline / (cfg.block // lanes))
-        build = 0.35
+        launch, build, strip, act = self.LINE_COST[self.precision]
 
-        def cost(k: int) -> float:
-            return math.ceil(lines * math.ceil(most / k) / (2 * SM_COUNT)) * (k + build)
+        def cost(shape: tuple) -> float:
+            lanes, strips = shape
+            parts = math.ceil(math.ceil(nline * lanes / cfg.block) / strips)
+            waves = math.ceil(lines * parts / (2 * SM_COUNT))
+            each = strip * spec.n_discrete_actions / 2 + act * spec.n_actions / lanes
+            return launch + waves * (build * nline / 1000 + strips * each)
 
-        strips = min((k for k in (1, 2, 4) if k <= max(1, most)), key=cost)
+        # in double precision more threads per state at least while the states
+        # do not fill the GPU (21,000 states: 1 / 2 / 4 threads 1.34 / 0.95 /
+        # 0.90 ms; 70,000: 1.55 / 1.63 / 1.77)
+        total = spec.n_states * n_items
+        least = 1 if self.precision == "fp32" else next((k for k, n in ((1, 60_000), (2, 30_000)) if total >= n), 4)
+        shapes = [(k, n) for k in (1, 2, 4, 8, 16) for n in (1, 2, 4)
+                  if k >= least and (k <= self.LINE_GROUP or scan >= 2 * k)  # (a group holds an action per thread)
+                  and n <= max(1, math.ceil(nline * k / cfg.block))]
+        lanes, strips = min(shapes, key=cost)
+        base, per = self.FULL_COST[self.precision]
+        if cost((lanes, strips)) > base + per * pairs / 1e6:
+            return full
+        if self.precision == "fp64" and nline <= cfg.block and scan < 20 * self.LINE_GROUP:
+            return full  # (the estimate is too low there: 128 x 150 x 372, 192 / 236; 200 x 150 x 238, 218 / 232)
         return dataclasses.replace(cfg, lanes=2 * lanes, sb=strips)
 
     def n_tiles(self) -> int:
