@@ -1127,7 +1127,7 @@ class RegimeKernels:
                   if k >= least and (k <= self.LINE_GROUP or scan >= 2 * k)  # (a group holds an action per thread)
                   and n <= max(1, math.ceil(nline * k / cfg.block))]
         lanes, strips = min(shapes, key=cost)
-        if pairs < 50_000:  # launches of 9 (full) to 17 us: single precision keeps skipping
+        if pairs < 200_000:  # launches of 9 (full) to 17 us: single precision keeps skipping
             return dataclasses.replace(cfg, lanes=2 * lanes, sb=strips)
         base, per = self.FULL_COST[self.precision]
         if cost((lanes, strips)) > base + per * pairs / 1e6:
