@@ -35,6 +35,7 @@ Reference semantics restated here: ``Q_and_F.py:138-168, 466-681, 1145-1209``,
 
 from __future__ import annotations
 
+import copy
 import dataclasses
 import hashlib
 import math
@@ -513,13 +514,35 @@ class RegimeKernels:
         self._layout()
         self._affine_all = self._affine_laws()
         self._affine = self._affine_all if precision == "fp32" else {}
+        self._search_plans()
+        self._set_tags()
+
+    def reshaped(self, cfg: LaunchConfig) -> RegimeKernels:
+        """The same regime and targets at another launch shape: layout and
+        laws are shared, and the search's plans unless their switches differ."""
+        new = copy.copy(self)
+        for k in ("_text", "src", "key", "module"):
+            new.__dict__.pop(k, None)
+        new.cfg = cfg
+        if dataclasses.replace(cfg, block=self.cfg.block, lanes=self.cfg.lanes, chunk=self.cfg.chunk, sb=self.cfg.sb,
+                               min_blocks=self.cfg.min_blocks) != self.cfg:
+            new._search_plans()
+        new._set_tags()
+        return new
+
+    def _search_plans(self) -> None:
         self._groups = self._group_plan()
         self._line = self._line_plan()
+        self._bnd = self._boundaries()
         if self._line is not None and not self._line_fits():
             self._line = None
+            self._bnd = self._boundaries()
+
+    def _set_tags(self) -> None:
         # kernel (a) carries the launch shape in its tag; the other kernels are
         # the same for every shape
-        what = (self.spec.name, [t.spec.name for t in self.targets], precision)
+        cfg = self.cfg
+        what = (self.spec.name, [t.spec.name for t in self.targets], self.precision)
         shape = cfg if self._line is None else dataclasses.replace(cfg, sb=1)  # (strips are an item word)
         name = self.spec.name.replace("-", "_") + "_"
         self.tag = name + hashlib.sha1(repr((*what, dataclasses.astuple(shape))).encode()).hexdigest()[:8]
@@ -594,14 +617,9 @@ class RegimeKernels:
         if tc:
             out.append(("rest", tc_header()))
         out.append(("both", _EXTRA_DEVICE))
-        part, lines = "both", []
-        for ln in self._bellman_source():
-            if ln.startswith("//@"):
-                out.append((part, "\n".join(lines)))
-                part, lines = ln[3:], []
-            else:
-                lines.append(ln)
-        out.append((part, "\n".join(lines)))
+        for k, text in enumerate(("\n" + "\n".join(self._bellman_source())).split("\n//@")):
+            part, _, text = text.partition("\n")
+            out.append((part if k else "both", text))
         parts: list[str] = []
         for t in self.targets:
             if not t.scalar and (t.needs_contraction or self.precision == "fp32"):
@@ -997,7 +1015,7 @@ class RegimeKernels:
     def _line_bytes(self, line: dict) -> int:
         """Shared memory of the line form: the whole continuous-action table,
         then the rows' windowed maxima and the rows."""
-        cols = self._boundaries()["A"]
+        cols = self._bnd["A"]
         value = 4 if self.precision == "fp32" else 8
         n_ac = self.spec.n_actions // self.spec.n_discrete_actions
         rows = max((x["coll"]["nob"] if x["coll"] else 1) * self.targets[ti].spec.states[x["pos"]].size
@@ -1110,13 +1128,13 @@ class RegimeKernels:
         scan = spec.actions[self._line["kscan"]].size
         lines = spec.n_states // nline * n_items
         launch, build, strip, act = self.LINE_COST[self.precision]
+        build, strip, act = build * nline / 1000, strip * spec.n_discrete_actions / 2, act * spec.n_actions
 
         def cost(shape: tuple) -> float:
             lanes, strips = shape
             parts = math.ceil(math.ceil(nline * lanes / cfg.block) / strips)
             waves = math.ceil(lines * parts / (2 * SM_COUNT))
-            each = strip * spec.n_discrete_actions / 2 + act * spec.n_actions / lanes
-            return launch + waves * (build * nline / 1000 + strips * each)
+            return launch + waves * (build + strips * (strip + act / lanes))
 
         # in double precision more threads per state at least while the states
         # do not fill the GPU (21,000 states: 1 / 2 / 4 threads 1.34 / 0.95 /
@@ -1314,7 +1332,7 @@ class RegimeKernels:
         det = self.tr.regime_id is not None and bool(self.targets)
         rid_phase = self._phase(self.tr.regime_id) if det else None
         unswitch = det and rid_phase in ("P", "D")
-        bnd = self._boundaries()
+        bnd = {k: list(v) for k, v in self._bnd.items()}
         bP, bD, bS, bSD, bA = bnd["P"], bnd["D"], bnd["S"], bnd["SD"], bnd["A"]
         if unswitch and id(self.tr.regime_id) not in {id(x) for x in bP + bD}:
             (bP if rid_phase == "P" else bD).append(self.tr.regime_id)

@@ -223,7 +223,7 @@ class SolveEngine:
         key = (spec.name, targets, cfg)
         rk = self._kernels.get(key)
         if rk is None:
-            rk = base if cfg == base.cfg else RegimeKernels(base.tr, [t.spec for t in base.targets], self.precision, cfg)
+            rk = base if cfg == base.cfg else base.reshaped(cfg)
             src = rk.source()
             rk.src = src
             rk.key = "lcm_" + hashlib.sha1(src.encode()).hexdigest()[:24]
