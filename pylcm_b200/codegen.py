@@ -1079,11 +1079,11 @@ class RegimeKernels:
     # us of a launch (B200, fitted to 63 grids x 2 to 4 batch sizes x 5 numbers
     # of threads, see line_config): (launch, build per 1000 nodes of the line,
     # strip, strip per action / threads) and of the full search (launch, per
-    # million pairs; for double precision 0.75 of the fit, so that a close call
+    # million pairs; for double precision 0.85 of the fit, so that a close call
     # stays with it, for single 1.08, where the search before the line form
     # was slower still)
     LINE_COST = {"fp32": (4.6, 7.5, 11.2, 0.039), "fp64": (8.9, 12.3, 8.3, 0.056)}
-    FULL_COST = {"fp32": (13.0, 2.8), "fp64": (12.3, 1.73)}
+    FULL_COST = {"fp32": (13.0, 2.8), "fp64": (14.0, 1.95)}
 
     def line_config(self, n_items: int) -> LaunchConfig:
         """The launch shape of kernel (a) for `n_items` instances where the
@@ -1130,28 +1130,42 @@ class RegimeKernels:
         launch, build, strip, act = self.LINE_COST[self.precision]
         build, strip, act = build * nline / 1000, strip * spec.n_discrete_actions / 2, act * spec.n_actions
 
-        def cost(shape: tuple) -> float:
-            lanes, strips = shape
-            parts = math.ceil(math.ceil(nline * lanes / cfg.block) / strips)
-            waves = math.ceil(lines * parts / (2 * SM_COUNT))
-            return launch + waves * (build + strips * (strip + act / lanes))
+        def waves(lanes: int, strips: int) -> int:
+            return math.ceil(lines * math.ceil(math.ceil(nline * lanes / cfg.block) / strips) / (2 * SM_COUNT))
+
+        def strips_of(lanes: int) -> int:
+            # a CTA that walks the whole line builds its rows once, more CTAs
+            # fill the last wave better: waves x (strips + build), the build
+            # worth a third of a strip (280 lines of 500: 2 strips 2.18, 1 strip
+            # 2.70 ms; 140 lines: 1.82, 1.55; 1792 lines, single precision: a
+            # batch's pass 29.8, 36.4)
+            most = max(1, math.ceil(nline * lanes / cfg.block))
+            return min((n for n in (1, 2, 4) if n <= most), key=lambda n: waves(lanes, n) * (n + 0.35))
+
+        def cost(lanes: int, strips: int) -> float:
+            return launch + waves(lanes, strips) * (build + strips * (strip + act / lanes))
 
         # in double precision more threads per state at least while the states
         # do not fill the GPU (21,000 states: 1 / 2 / 4 threads 1.34 / 0.95 /
         # 0.90 ms; 70,000: 1.55 / 1.63 / 1.77)
         total = spec.n_states * n_items
         least = 1 if self.precision == "fp32" else next((k for k, n in ((1, 60_000), (2, 30_000)) if total >= n), 4)
-        shapes = [(k, n) for k in (1, 2, 4, 8, 16) for n in (1, 2, 4)
-                  if k >= least and (k <= self.LINE_GROUP or scan >= 2 * k)  # (a group holds an action per thread)
-                  and n <= max(1, math.ceil(nline * k / cfg.block))]
-        lanes, strips = min(shapes, key=cost)
+        shapes = [(k, strips_of(k)) for k in (1, 2, 4, 8, 16)
+                  if k >= least and (k <= self.LINE_GROUP or scan >= 2 * k)]  # (a group holds an action per thread)
+        lanes, strips = min(shapes, key=lambda x: cost(*x))
         if pairs < 200_000:  # launches of 9 (full) to 17 us: single precision keeps skipping
             return dataclasses.replace(cfg, lanes=2 * lanes, sb=strips)
         base, per = self.FULL_COST[self.precision]
-        if cost((lanes, strips)) > base + per * pairs / 1e6:
+        if cost(lanes, strips) > base + per * pairs / 1e6:
             return full
-        if self.precision == "fp64" and nline <= cfg.block and scan < 20 * self.LINE_GROUP:
-            return full  # (the estimate is too low there: 128 x 150 x 372, 192 / 236; 200 x 150 x 238, 218 / 232)
+        if self.precision == "fp64":
+            # where the estimate is too low (full search / line form, us): few
+            # actions, unless long lines fill their strips (128 x 150 x 372,
+            # 192 / 236; 800 x 150 x 60, 206 / 262; 500 x 150 x 95, 238 / 183),
+            # and the shortest lines (24 x 800 x 74, 56 / 72)
+            held = math.ceil(nline * lanes / cfg.block) * cfg.block // lanes
+            if nline < 32 or (scan < 20 * self.LINE_GROUP and (nline <= cfg.block or nline < 0.85 * held)):
+                return full
         return dataclasses.replace(cfg, lanes=2 * lanes, sb=strips)
 
     def n_tiles(self) -> int:
