@@ -1603,7 +1603,8 @@ class RegimeKernels:
                     rows = [] if multi else [("row", off)] + ([("rowh", off_hi)] if off_hi is not None else [])
                     if coll is not None and ti == coll["ti"]:
                         rows = []
-                        inner.append(f"{T} ev = lcm_interp1s{'f' if fast else ''}<{T}>(AF.R, C.n{ti}_{coll['posA']}, c{coll['ca']});")
+                        read = "lcm_interp1sf" if fast else "lcm_interp1s" if line is None else "lcm_interp1sl"
+                        inner.append(f"{T} ev = {read}<{T}>(AF.R, C.n{ti}_{coll['posA']}, c{coll['ca']});")
                     if multi:
                         inner.append(f"{T} ev = ({T})0;")
                         inner += self._sim_extrapolated_expectation(ti, t, T, E, None, proc_names, dn, mk)
