@@ -3384,7 +3384,7 @@ class RegimeKernels:
         # words, values, weights); at 10^5 columns with J = K = 32 the FP64
         # products.  So a thread reads its column's values before the weights
         # are made (up to 16 nodes, or the first chunk of 8), two weights per
-        # shared-memory read, and 16 rows at a time (three CTAs per SM).  A
+        # shared-memory read, and up to 16 rows at a time.  A
         # value of -inf or NaN (an infeasible state; one lane of a warp is enough
         # to send it the slow way) is taken out of the sums as a bit and put
         # back at the end: the sum is -inf or NaN in every row that weighs it.
@@ -3394,7 +3394,15 @@ class RegimeKernels:
         # columns 99 -> 86, 16 x 81,000 30 -> 22 (with the reads but without
         # the bits).
         B = 256
-        KC = min(K, 16)
+        # The rows of a pass are dealt evenly (of 17 rows at 16 a time the second
+        # pass works on 15 that are not there: 31 us where 33 at a time took 23
+        # and 9 take 21), and an odd number of values held in registers takes 8
+        # (13 x 13, 100,000 columns: 32 us in one pass, 19 in two; 22 with 33
+        # rows at a time).  An odd row's last pair needs no test: the weight
+        # beyond it is 0 (49 x 49, 480 columns: 143 us with one, 80 without).
+        # Three CTAs per SM from 9 rows on (16 x 16: 17 -> 18 us at 480 columns,
+        # 29 -> 23 at 100,000).
+        KC = math.ceil(K / math.ceil(K / (8 if J <= 16 and J % 2 else 16)))
         JC = J if J <= 16 else 8
         one = JC == J  # every value stays in registers
         # rows of W start on 16 bytes (where the static 48 KB hold them padded)
@@ -3413,7 +3421,7 @@ class RegimeKernels:
         self.e_words = 9 + len(tg.states)
         ap(f"// ---- expectation {spec.name} -> {tg.name}: K={K} J={J}")
         ap(
-            f'extern "C" __global__ void __launch_bounds__({B}{', 3' if K > 16 else ''}) {name}('
+            f'extern "C" __global__ void __launch_bounds__({B}{', 3' if K > 8 else ''}) {name}('
             "const i64* __restrict__ items, const int* __restrict__ tile_prefix, int n_items, int n_tiles) {"
         )
         ap(f"  __shared__ __align__(16) double W[{K * JS}];")
@@ -3469,6 +3477,8 @@ class RegimeKernels:
             ap("    if (threadIdx.x == 0) Wodd = 0;")
         for s_ in self._weight_fill(t, B, JS):
             ap("    " + s_)
+        if JS > J:
+            ap(f"    for (int k = threadIdx.x; k < {K}; k += {B}) W[k * {JS} + {J}] = 0.0;")
         ap("    __syncthreads();")
         ap(f"    for (int k = threadIdx.x; k < {K}; k += {B}) {{")
         if bits:
@@ -3508,18 +3518,19 @@ class RegimeKernels:
         ap("          }")
         ap("          if (fin) {")
         ap(f"            #pragma unroll\n            for (int q = 0; q < {JC}; q += 2) {{")
+        ap(f"              if (j0 + q >= {J}) break;")
         ap(f"              #pragma unroll\n              for (int kk = 0; kk < {KC}; ++kk) {{")
         ap(f"                const int k = k0 + kk; if (k >= {K}) continue;")
-        ap(f"                if ({int(pair)} && q + 1 < {JC} && j0 + q + 1 < {J}) {{")
-        ap(f"                  const double2 w = *reinterpret_cast<const double2*>(&W[k * {JS} + j0 + q]);")
-        ap("                  acc[kk] = __dadd_rn(acc[kk], __dmul_rn(w.x, v[q]));")
-        ap(f"                  acc[kk] = __dadd_rn(acc[kk], __dmul_rn(w.y, v[q + 1 < {JC} ? q + 1 : q]));")
-        ap("                } else {")
-        ap("                  #pragma unroll")
-        ap(f"                  for (int r = q; r < q + 2; ++r)")
-        ap(f"                    if (r < {JC} && j0 + r < {J})")
-        ap(f"                      acc[kk] = __dadd_rn(acc[kk], __dmul_rn(W[k * {JS} + j0 + r], v[r < {JC} ? r : q]));")
-        ap("                }")
+        if pair:
+            # (an odd row's last pair: weight and value beyond it are 0)
+            ap(f"                const double2 w = *reinterpret_cast<const double2*>(&W[k * {JS} + j0 + q]);")
+            ap("                acc[kk] = __dadd_rn(acc[kk], __dmul_rn(w.x, v[q]));")
+            ap(f"                if (q + 1 < {JC}) acc[kk] = __dadd_rn(acc[kk], __dmul_rn(w.y, v[q + 1 < {JC} ? q + 1 : q]));")
+        else:
+            ap("                #pragma unroll")
+            ap("                for (int r = q; r < q + 2; ++r)")
+            ap(f"                  if (r < {JC} && j0 + r < {J})")
+            ap(f"                    acc[kk] = __dadd_rn(acc[kk], __dmul_rn(W[k * {JS} + j0 + r], v[r < {JC} ? r : q]));")
         ap("              }")
         ap("            }")
         ap("          } else {  // zero weights ignore a value that is not finite")
