@@ -186,6 +186,12 @@ class Server:
     # Regimes with two continuous states keep the search by collapsed rows: NaN
     # values make the line form the slower one over long horizons
     SHAPE = LaunchConfig(block=256, lanes=2, chunk=512, sb=2, line_axes=1)
+    # in double precision from this many points of the longest continuous action
+    # on; below, the full search (B200, us of three periods' launches, full
+    # search / line form: 1000 wealth points x 60 actions x 32 requests 363 /
+    # 638, x 200 974 / 859, x 500 2452 / 1219; 100 x 60, x 200, x 500, 64
+    # requests: 138 / 261, 355 / 466, 828 / 888)
+    LINE_ACTIONS_FP64 = 256
 
     def __init__(self, device: int = 0, precision: str = "fp32", max_batch: int = 32, n_streams: int = 4,
                  hbm_budget_bytes: int | None = None, configs: Mapping | None = None, pool_slots: int = 4,
@@ -241,11 +247,18 @@ class Server:
                 cfgs.update(self.configs.get(req.family, {}))
                 for s in req.model.regime_specs:
                     if s.name not in cfgs:
-                        cfgs[s.name] = self.SHAPE
+                        cfgs[s.name] = self.shape(s)
                 self._family_cfg[req.family] = cfgs
             eng = SolveEngine(req.model, self.precision, configs=cfgs, device=self.device)
             self._engines[req.key] = eng
         return eng
+
+    def shape(self, spec) -> LaunchConfig:
+        """The launch shape of a regime that is neither tuned nor given."""
+        longest = max((a.size for a in spec.actions if a.kind == "continuous"), default=0)
+        if self.precision == "fp64" and longest < self.LINE_ACTIONS_FP64:
+            return dataclasses.replace(self.SHAPE, line_axes=0)
+        return self.SHAPE
 
     @staticmethod
     def _n_agents(req: Request) -> int:
